@@ -8,9 +8,9 @@
 // Additions, subtractions and the wide reduction use PTX carry chains
 // (add.cc / addc / sub.cc / subc / mad.lo.cc / madc.hi.cc); each chain is a run
 // of consecutive volatile asm statements with no other instruction between
-// them touching the condition code.  The Montgomery product is CIOS written as
-// 64-bit multiply-adds, which a throughput probe measured faster than the
-// carry-chain form.
+// them touching the condition code.  The Montgomery product keeps its running
+// value as two sums of 64-bit columns so that each word product is one wide
+// multiply-add.
 #pragma once
 
 #include <cstdint>
@@ -157,58 +157,10 @@ namespace hmpc_gb300
         mod_sub<L>(r, z, a, m);
     }
 
-    // Montgomery product r = a*b*R^{-1} mod Q, a, b < Q: coarsely integrated
-    // operand scanning with one word of headroom; the result is fully reduced,
-    // which is what hmpc's schoolbook + separated REDC yields
-    // (hmpc/ints/mod.hpp:41-46, hmpc/core/num/modulo.hpp:30-66).
-    //
-    // The word products are written as 64-bit multiply-adds
-    // (a_j * b_i + t_j + carry fits 64 bits), which the compiler maps to wide
-    // integer multiply-adds with a 64-bit addend.  Measured on GB300 for
-    // L = 8 this runs 1.20x faster than the same algorithm written as
-    // explicit mad.lo.cc / madc.hi.cc carry chains (51.9 vs 43.2 G
-    // products/s in a throughput probe), because each chained multiply-add
-    // otherwise costs an extra carry instruction on the ALU pipe.
+    // r = t mod Q for t = t[0..L] < 2Q: subtract Q once if t >= Q
     template<int L>
-    __device__ __forceinline__ void mont_mul(uint32_t (&r)[L], const uint32_t (&a)[L], const uint32_t (&b)[L],
-                                             const Modulus<L>& m)
+    __device__ __forceinline__ void reduce_once(uint32_t (&r)[L], const uint32_t (&t)[L + 1], const Modulus<L>& m)
     {
-        uint32_t t[L + 2];
-#pragma unroll
-        for (int j = 0; j < L + 2; ++j)
-        {
-            t[j] = 0u;
-        }
-#pragma unroll
-        for (int i = 0; i < L; ++i)
-        {
-            // t += a * b_i
-            uint64_t c = 0;
-#pragma unroll
-            for (int j = 0; j < L; ++j)
-            {
-                const uint64_t s = static_cast<uint64_t>(a[j]) * b[i] + t[j] + c;
-                t[j] = static_cast<uint32_t>(s);
-                c = s >> 32;
-            }
-            uint64_t s = static_cast<uint64_t>(t[L]) + c;
-            t[L] = static_cast<uint32_t>(s);
-            t[L + 1] = static_cast<uint32_t>(s >> 32);
-            // t = (t + (t_0 * N') * Q) / 2^32
-            const uint32_t mq = t[0] * m.ninv;
-            c = (static_cast<uint64_t>(mq) * m.q[0] + t[0]) >> 32;
-#pragma unroll
-            for (int j = 1; j < L; ++j)
-            {
-                const uint64_t u = static_cast<uint64_t>(mq) * m.q[j] + t[j] + c;
-                t[j - 1] = static_cast<uint32_t>(u);
-                c = u >> 32;
-            }
-            s = static_cast<uint64_t>(t[L]) + c;
-            t[L - 1] = static_cast<uint32_t>(s);
-            t[L] = t[L + 1] + static_cast<uint32_t>(s >> 32);
-        }
-        // t < 2Q: subtract Q once if t >= Q
         uint32_t d[L];
         d[0] = ptx::sub_cc(t[0], m.q[0]);
 #pragma unroll
@@ -216,12 +168,178 @@ namespace hmpc_gb300
         {
             d[j] = ptx::subc_cc(t[j], m.q[j]);
         }
-        uint32_t borrow = ptx::subc(t[L], 0u);
+        const uint32_t borrow = ptx::subc(t[L], 0u);
 #pragma unroll
         for (int j = 0; j < L; ++j)
         {
             r[j] = borrow ? t[j] : d[j];
         }
+    }
+
+    // A value of L + 2 words held as two sums of 64-bit columns: `even` covers
+    // words 0..EW-1 (columns at words 0, 2, ...), `odd` words 1..OW (columns
+    // at words 1, 3, ...), EW and OW being L and L - 1 rounded up and down to
+    // whole columns, and `top` is the count at word L + 1.  A word product
+    // a_j * b lies exactly on one 64-bit column, so a row of products is two
+    // chains of mad.lo.cc / madc.hi.cc pairs over adjacent words; each pair is
+    // one wide multiply-add with carry in and out, where a single running sum
+    // needs a further addition for each product.
+    template<int L>
+    struct Columns
+    {
+        static constexpr int EW = (L + 1) / 2 * 2;
+        static constexpr int OW = L / 2 * 2;
+        uint32_t even[EW];
+        uint32_t odd[OW < 2 ? 2 : OW];
+        uint32_t top;
+        uint32_t pending;  // added at word 0 by the next row
+
+        // even / odd = a * b
+        __device__ __forceinline__ void set_product(const uint32_t (&a)[L], uint32_t b)
+        {
+#pragma unroll
+            for (int j = 0; j < L; ++j)
+            {
+                const uint64_t w = static_cast<uint64_t>(a[j]) * b;
+                uint32_t* column = j % 2 ? odd + (j - 1) : even + j;
+                column[0] = static_cast<uint32_t>(w);
+                column[1] = static_cast<uint32_t>(w >> 32);
+            }
+            top = 0u;
+            pending = 0u;
+        }
+
+        // += a * b (+ pending at word 0 when First).  The odd chain goes first:
+        // it starts at word 1, where the carry of the pending word's addition
+        // belongs.
+        template<bool First>
+        __device__ __forceinline__ void add_product(const uint32_t (&a)[L], uint32_t b)
+        {
+            if constexpr (First)
+            {
+                even[0] = ptx::add_cc(even[0], pending);
+            }
+            if constexpr (L > 1)
+            {
+                odd[0] = First ? ptx::madc_lo_cc(a[1], b, odd[0]) : ptx::mad_lo_cc(a[1], b, odd[0]);
+                odd[1] = ptx::madc_hi_cc(a[1], b, odd[1]);
+#pragma unroll
+                for (int j = 3; j < L; j += 2)
+                {
+                    odd[j - 1] = ptx::madc_lo_cc(a[j], b, odd[j - 1]);
+                    odd[j] = ptx::madc_hi_cc(a[j], b, odd[j]);
+                }
+            }
+            // the odd chain ends at word L + 1 (even L) or L (odd L)
+            if constexpr (L % 2 == 0)
+            {
+                top = ptx::addc(top, 0u);
+            }
+            else if constexpr (L > 1 || First)
+            {
+                even[L] = ptx::addc_cc(even[L], 0u);
+                top = ptx::addc(top, 0u);
+            }
+            even[0] = ptx::mad_lo_cc(a[0], b, even[0]);
+            even[1] = ptx::madc_hi_cc(a[0], b, even[1]);
+#pragma unroll
+            for (int j = 2; j < L; j += 2)
+            {
+                even[j] = ptx::madc_lo_cc(a[j], b, even[j]);
+                even[j + 1] = ptx::madc_hi_cc(a[j], b, even[j + 1]);
+            }
+            // the even chain ends at word L (even L) or L + 1 (odd L)
+            if constexpr (L % 2 == 0)
+            {
+                odd[L - 1] = ptx::addc_cc(odd[L - 1], 0u);
+            }
+            top = ptx::addc(top, 0u);
+        }
+
+        // / 2^32, word 0 being zero: word k becomes word k - 1, so the two
+        // column sums change places; the even sum's word 1 is left over
+        __device__ __forceinline__ void shift()
+        {
+            uint32_t e[EW], o[OW < 2 ? 2 : OW];
+            pending = even[1];
+#pragma unroll
+            for (int j = 0; j < EW; ++j)
+            {
+                e[j] = j < OW ? odd[j] : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < OW; ++j)
+            {
+                o[j] = j + 2 < EW ? even[j + 2] : 0u;
+            }
+            (L % 2 == 0 ? o[L > 1 ? L - 1 : 0] : e[L % 2 ? L : 0]) = top;
+            top = 0u;
+#pragma unroll
+            for (int j = 0; j < EW; ++j)
+            {
+                even[j] = e[j];
+            }
+#pragma unroll
+            for (int j = 0; j < OW; ++j)
+            {
+                odd[j] = o[j];
+            }
+        }
+
+        // words 0..L of the value, which is below 2^(32(L+1))
+        __device__ __forceinline__ void value(uint32_t (&t)[L + 1]) const
+        {
+            t[0] = ptx::add_cc(even[0], pending);
+#pragma unroll
+            for (int j = 1; j < L; ++j)
+            {
+                t[j] = ptx::addc_cc(even[j], odd[j - 1]);
+            }
+            t[L] = ptx::addc(L % 2 ? even[L % 2 ? L : 0] : odd[L > 1 ? L - 1 : 0], 0u);
+        }
+    };
+
+    // Montgomery product r = a*b*R^{-1} mod Q, a, b < Q, fully reduced, which is
+    // what hmpc's schoolbook + separated REDC yields (hmpc/ints/mod.hpp:41-46,
+    // hmpc/core/num/modulo.hpp:30-66): operand scanning, each row a * b_i and
+    // the multiple of Q that clears word 0, on 64-bit columns (Columns).
+    //
+    // Bound by the wide integer multiply-add, of which it needs 2L^2 + L: on a
+    // GB300 71.3 G products/s at L = 8 (9.7 T multiply-adds/s, 31 per SM and
+    // clock), 249 G/s at L = 4.  The same rows as one running sum of 64-bit
+    // multiply-adds reach 52.6 and 197 G/s: every product then needs two more
+    // additions.  One limb has no chain to shorten and is slower on columns
+    // (1.92 against 2.18 T/s), so it keeps the running sum.
+    template<int L>
+    __device__ __forceinline__ void mont_mul(uint32_t (&r)[L], const uint32_t (&a)[L], const uint32_t (&b)[L],
+                                             const Modulus<L>& m)
+    {
+        uint32_t t[L + 1];
+        if constexpr (L == 1)
+        {
+            const uint64_t ab = static_cast<uint64_t>(a[0]) * b[0];
+            const uint32_t mq = static_cast<uint32_t>(ab) * m.ninv;
+            const uint64_t c = (static_cast<uint64_t>(mq) * m.q[0] + static_cast<uint32_t>(ab)) >> 32;
+            const uint64_t s = (ab >> 32) + c;
+            t[0] = static_cast<uint32_t>(s);
+            t[1] = static_cast<uint32_t>(s >> 32);
+        }
+        else
+        {
+            Columns<L> c;
+            c.set_product(a, b[0]);
+            c.template add_product<false>(m.q, c.even[0] * m.ninv);
+            c.shift();
+#pragma unroll
+            for (int i = 1; i < L; ++i)
+            {
+                c.template add_product<true>(a, b[i]);
+                c.template add_product<false>(m.q, c.even[0] * m.ninv);
+                c.shift();
+            }
+            c.value(t);
+        }
+        reduce_once<L>(r, t, m);
     }
 
     // Reduction of a W-word value with R' = 2^(32W) (hmpc/core/num/modulo.hpp
