@@ -137,11 +137,6 @@ namespace hmpc_gb300::detail
             return fail(HMPC_ERROR_INVALID_ARGUMENT, "tensor producer without source");
         }
         const int log_n = __builtin_ctzll(n);
-        if (log_n < mod->kt->radix_bits && !poly_rng)
-        {
-            // fewer stages than one register group holds: the per-stage kernel
-            return run_plain(ctx, mod, n, batch, inverse, kind, vx2, security, src, out);
-        }
         hmpc_modulus::TileChoice choice;
         {
             std::lock_guard<std::mutex> lock(mod->tables_mutex);
@@ -203,42 +198,32 @@ namespace hmpc_gb300::detail
             }
             choice = hmpc_modulus::TileChoice{};
         }
-        PlanOptions options;
-        options.max_local_bits = choice.local_bits;
-        options.col_bits = choice.col_bits;
-        const std::vector<PassPlan> plan = plan_transform(L, log_n, batch, inverse, choice.radix_bits, options);
-        const RngKey rng = ctx->rng();
-        // A pass after the first whose grid fills at most a quarter of the SMs
-        // (single polynomials: the launch gap is a large share of its time)
-        // launches with programmatic dependence on the pass before: 87.5 ->
-        // 84.9 us for one polynomial of 2^15 coefficients at 8 limbs, while
-        // 16 polynomials measured 2 % slower that way.  Ordinary launches
-        // while the stream is being captured.
+        // Every pass launches with programmatic dependence on the kernel before
+        // it in the stream: its CTAs take the SMs' free slots and fetch their
+        // first twiddles while that kernel drains, and wait for its completion
+        // before reading an element.  Measured over the passes of one call:
+        // 20.9 -> 14.9 us (one polynomial of 2^15 at 8 limbs), 18.8 -> 16.2 us
+        // (12 of 2^13 at 6), 297.3 -> 295.2 us (64 of 2^15 at 8): never slower.
+        // Ordinary launches while the stream is being captured.
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         const bool capturing =
             cudaStreamIsCapturing(ctx->stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone;
-        if (!ctx->sm_count)
-        {
-            HMPC_CUDA(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device),
-                      "querying the SM count");
-        }
+        const std::vector<PairPlan> plan = plan_pairs(L, log_n, batch, inverse, choice.local_bits, choice.col_bits);
         for (size_t i = 0; i < plan.size(); ++i)
         {
-            NttPassParams p = plan[i].params;
-            p.dependent = i > 0 && !capturing && 4ull * plan[i].grid <= static_cast<uint64_t>(ctx->sm_count) ? 1u : 0u;
+            PairPassParams p = plan[i].params;
+            p.dependent = capturing ? 0u : 1u;
             p.out = out;
             p.src = i == 0 ? src : nullptr;
             p.twiddles = inverse ? t->inverse : t->forward;
             p.small_table = mod->small_table;
             p.elements = n * batch;
-            p.rng = rng;
+            p.rng = ctx->rng();
             p.vx2 = vx2;
             p.top_mask = top_mask;
             p.poly_rng = poly_rng;
             p.rng_slot = rng_slot;
-            const int k = i == 0 ? kind : producer_tensor;
-            cudaError_t e = mod->kt->ntt_pass(p, k, k == producer_tensor ? 1 : nw, choice.radix_bits, mod->h,
-                                              plan[i].grid,
+            cudaError_t e = mod->kt->ntt_pair(p, i == 0 ? kind : producer_tensor, nw, inverse, mod->h, plan[i].grid,
                                               plan[i].block, plan[i].smem, ctx->stream);
             if (e != cudaSuccess)
             {
@@ -784,7 +769,7 @@ int hmpc_modulus_set_plan(hmpc_modulus* mod, uint64_t n, uint64_t batch, int inv
     }
     else if ((radix_bits != 2 && radix_bits != 3) || local_bits < 0 || local_bits > 13 || col_bits < 0 ||
              col_bits > 6 ||
-             (local_bits && static_cast<uint64_t>(mod->c.limbs) * 4u * smem_words(1u << local_bits) > 200 * 1024))
+             (local_bits && static_cast<uint64_t>(mod->c.limbs) * 4u * ((33u << local_bits) >> 5) > 200 * 1024))
     {
         return fail(HMPC_ERROR_INVALID_ARGUMENT, "tile shape out of range");
     }
@@ -830,8 +815,6 @@ int hmpc_modulus_tune(hmpc_modulus* mod, uint64_t n, uint64_t batch, int inverse
     cudaEventCreate(&t1);
     const int log_n = __builtin_ctzll(n);
     const auto key = std::make_tuple(log_n, inverse ? 1 : 0, batch);
-    PlanOptions def;
-    const int b0 = local_bits_for(L, def);
     float best = 1e30f;
     hmpc_modulus::TileChoice best_choice;
     auto time_choice = [&](const hmpc_modulus::TileChoice& choice) {
@@ -887,22 +870,15 @@ int hmpc_modulus_tune(hmpc_modulus* mod, uint64_t n, uint64_t batch, int inverse
             best_choice = cluster;
         }
     }
-    for (int R : {3, 2})
+    for (int tile_bits = 7; tile_bits <= 10; ++tile_bits)
     {
-        for (int lb = std::max(R + 2, b0 - 5); lb <= std::min(13, b0 + 1); ++lb)
+        for (int c : {2, 3, 4})
         {
-            if (static_cast<uint64_t>(L) * 4u * smem_words(1u << lb) > 200 * 1024)
+            const float sample = time_choice({3, tile_bits, c});
+            if (sample < best)
             {
-                continue;
-            }
-            for (int c : {3, 4, 5})
-            {
-                const float sample = time_choice({R, lb, c});
-                if (sample < best)
-                {
-                    best = sample;
-                    best_choice = {R, lb, c};
-                }
+                best = sample;
+                best_choice = {3, tile_bits, c};
             }
         }
     }
@@ -1370,7 +1346,7 @@ int hmpc_lhe_keygen(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_
         std::lock_guard<std::mutex> lock(q->tables_mutex);
         auto it = q->tile_choices.find(std::make_tuple(__builtin_ctzll(n), 0, static_cast<uint64_t>(1)));
         const int radix = it == q->tile_choices.end() ? hmpc_modulus::TileChoice{}.radix_bits : it->second.radix_bits;
-        fork = radix != 0 && __builtin_ctzll(n) >= q->kt->radix_bits;
+        fork = radix != 0;
     }
     fork = fork && ctx->aux();
     if (fork)

@@ -1,7 +1,7 @@
 // Batched transforms of polynomials of uneven degree: one persistent kernel
 // launch per batch, replayed from a captured CUDA graph, with the tile shape
-// (register radix, stages per shared-memory pass, coalescing columns) chosen
-// by timing candidates on the device.
+// (stages per pass, coalescing columns) chosen by timing candidates on the
+// device.
 #include <algorithm>
 #include <cstring>
 #include <numeric>
@@ -28,12 +28,13 @@ struct hmpc_ntt_batch
     float tuned_ms = 0.f;
 
     // plan
-    std::vector<NttPassParams> params;        // host copy (pointers rebound per run)
+    std::vector<PairPassParams> params;        // host copy (pointers rebound per run)
     std::vector<uint32_t> param_poly;         // params index -> polynomial
     std::vector<uint32_t> param_pass;         // params index -> pass
     uint32_t items = 0;
     size_t smem = 0;
     unsigned grid = 0;
+    unsigned block = 0;
     std::vector<uint32_t> item_wait_host, item_signal_host;
     // polls of a wait before it gives up, and the test hook's withheld item
     // (1-based, 0: none; hmpc_ntt_batch_set_test_wait)
@@ -41,10 +42,10 @@ struct hmpc_ntt_batch
     uint32_t withheld = 0;
 
     // device state
-    NttPassParams* d_params = nullptr;
+    PairPassParams* d_params = nullptr;
     uint32_t* d_items = nullptr;               // 5 arrays of `items` words
     uint32_t* d_counters = nullptr;            // one per polynomial + control block
-    NttPassParams* h_params = nullptr;         // pinned staging
+    PairPassParams* h_params = nullptr;         // pinned staging
     cudaStream_t stream = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t start = nullptr, finish = nullptr;
@@ -276,23 +277,20 @@ struct hmpc_ntt_batch
     }
 
     // Build the work list and device arrays for one configuration.
-    int build(int R, int b, int c_pref)
+    int build(int b, int c_pref)
     {
         release_plan();
-        radix_bits = R;
+        radix_bits = 3;
         local_bits = b;
         col_bits = c_pref;
         const int L = mod->c.limbs;
-        PlanOptions o;
-        o.max_local_bits = b;
-        o.col_bits = c_pref;
-        o.spread_small_batches = false;
+        block = std::max(32u, 1u << (b - 1));
+        smem = 2ull * static_cast<size_t>(L) * block * sizeof(uint32_t);
         params.clear();
         param_poly.clear();
         param_pass.clear();
-        std::vector<std::vector<PassPlan>> plans(degrees.size());
+        std::vector<std::vector<PairPlan>> plans(degrees.size());
         size_t max_passes = 0;
-        smem = 0;
         for (size_t i = 0; i < degrees.size(); ++i)
         {
             Tables* t = nullptr;
@@ -300,16 +298,8 @@ struct hmpc_ntt_batch
             {
                 return rc;
             }
-            plans[i] = plan_transform(L, __builtin_ctzll(degrees[i]), 1, inverse, R, o);
+            plans[i] = plan_pairs(L, __builtin_ctzll(degrees[i]), 1, inverse, b, c_pref, block);
             max_passes = std::max(max_passes, plans[i].size());
-            for (const PassPlan& pp : plans[i])
-            {
-                smem = std::max(smem, pp.smem);
-            }
-        }
-        if (smem > 200 * 1024)
-        {
-            return fail(HMPC_ERROR_UNSUPPORTED, "tile configuration exceeds shared memory");
         }
         // params index of (poly, pass); items: every pass-0 item first, larger
         // polynomials first, then pass 1, ...
@@ -320,7 +310,7 @@ struct hmpc_ntt_batch
             mod->prepare(degrees[i], &t);
             for (size_t k = 0; k < plans[i].size(); ++k)
             {
-                NttPassParams p = plans[i][k].params;
+                PairPassParams p = plans[i][k].params;
                 p.twiddles = inverse ? t->inverse : t->forward;
                 p.small_table = mod->small_table;
                 p.elements = degrees[i];
@@ -363,7 +353,7 @@ struct hmpc_ntt_batch
         item_wait_host = item_wait;
         item_signal_host = item_signal;
         withheld = 0;
-        const size_t pbytes = params.size() * sizeof(NttPassParams);
+        const size_t pbytes = params.size() * sizeof(PairPassParams);
         HMPC_CUDA(cudaMalloc(&d_params, pbytes), "allocating batch parameters");
         HMPC_CUDA(cudaMallocHost(&h_params, pbytes), "allocating batch parameters");
         std::memcpy(h_params, params.data(), pbytes);
@@ -378,7 +368,7 @@ struct hmpc_ntt_batch
                   "uploading work list");
         int sms = 0;
         HMPC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device), "querying SMs");
-        const int per_sm = std::max(1, mod->kt->ntt_batched_blocks_per_sm(R, smem));
+        const int per_sm = std::max(1, mod->kt->ntt_batched_blocks_per_sm(inverse, block, smem));
         grid = static_cast<unsigned>(std::min<uint64_t>(items, static_cast<uint64_t>(sms) * per_sm));
         return capture();
     }
@@ -407,7 +397,7 @@ struct hmpc_ntt_batch
         cudaError_t e = cudaMemsetAsync(d_counters, 0, (degrees.size() + 4) * sizeof(uint32_t), stream);
         if (e == cudaSuccess)
         {
-            e = mod->kt->ntt_batched(bp, radix_bits, mod->h, grid, smem, stream);
+            e = mod->kt->ntt_batched(bp, inverse, mod->h, grid, block, smem, stream);
         }
         cudaError_t e2 = cudaStreamEndCapture(stream, &graph);
         if (e != cudaSuccess || e2 != cudaSuccess)
@@ -507,7 +497,7 @@ struct hmpc_ntt_batch
             h_params[k].out = out[i];
             h_params[k].src = param_pass[k] == 0 ? in[i] : nullptr;
         }
-        HMPC_CUDA(cudaMemcpyAsync(d_params, h_params, params.size() * sizeof(NttPassParams), cudaMemcpyHostToDevice,
+        HMPC_CUDA(cudaMemcpyAsync(d_params, h_params, params.size() * sizeof(PairPassParams), cudaMemcpyHostToDevice,
                                   stream),
                   "uploading batch pointers");
         bound_in.assign(in, in + degrees.size());
@@ -610,9 +600,7 @@ int hmpc_ntt_batch_create(hmpc_context* ctx, hmpc_modulus* mod, uint64_t count, 
         return cuda_fail(e, "creating the batch stream");
     }
     const int L = mod->c.limbs;
-    PlanOptions def;
-    const int b_default = local_bits_for(L, def);
-    int best_r = 3, best_b = b_default, best_c = 4;
+    int best_r = 3, best_b = 9, best_c = 3;
     if (autotune == HMPC_BATCH_TENSOR_CORES)
     {
         if (!b->tc_covers())
@@ -644,28 +632,21 @@ int hmpc_ntt_batch_create(hmpc_context* ctx, hmpc_modulus* mod, uint64_t count, 
         float best = 1e30f;
         if (ok)
         {
-            for (int R : {3, 2})
+            for (int tile_bits = 7; tile_bits <= 10; ++tile_bits)
             {
-                for (int lb : {b_default - 1, b_default, b_default + 1})
+                for (int c : {2, 3, 4})
                 {
-                    for (int c : {3, 4, 5})
+                    if (b->build(tile_bits, c) != HMPC_OK)
                     {
-                        if (lb < 8 || static_cast<uint64_t>(L) * 4u * smem_words(1u << lb) > 200 * 1024)
-                        {
-                            continue;
-                        }
-                        if (b->build(R, lb, c) != HMPC_OK)
-                        {
-                            continue;
-                        }
-                        const float ms = time_config(b, ins, bufs);
-                        if (ms < best)
-                        {
-                            best = ms;
-                            best_r = R;
-                            best_b = lb;
-                            best_c = c;
-                        }
+                        continue;
+                    }
+                    const float ms = time_config(b, ins, bufs);
+                    if (ms < best)
+                    {
+                        best = ms;
+                        best_r = 3;
+                        best_b = tile_bits;
+                        best_c = c;
                     }
                 }
             }
@@ -693,7 +674,7 @@ int hmpc_ntt_batch_create(hmpc_context* ctx, hmpc_modulus* mod, uint64_t count, 
         }
         b->tuned_ms = best < 1e29f ? best : 0.f;
     }
-    if (int rc = best_r == 0 ? b->build_tc(best_b) : b->build(best_r, best_b, best_c))
+    if (int rc = best_r == 0 ? b->build_tc(best_b) : b->build(best_b, best_c))
     {
         delete b;
         return rc;

@@ -11,6 +11,7 @@
 #include "cluster.cuh"
 #include "linalg.cuh"
 #include "ntt.cuh"
+#include "pair.cuh"
 #include "plain.cuh"
 #include "tensor_ntt.cuh"
 
@@ -46,8 +47,6 @@ namespace hmpc_gb300
 
     struct KernelTable
     {
-        cudaError_t (*ntt_pass)(const NttPassParams& p, int kind, int nw, int radix_bits, const HostModulus& m,
-                                unsigned grid, unsigned block, size_t smem, cudaStream_t stream);
         cudaError_t (*fma)(uint32_t* d, const uint32_t* a, const uint32_t* b, const uint32_t* c, uint64_t elements,
                            const HostModulus& m, cudaStream_t stream);
         cudaError_t (*binary)(uint32_t* out, const uint32_t* a, uint64_t a_elements, const uint32_t* b,
@@ -74,11 +73,10 @@ namespace hmpc_gb300
         cudaError_t (*dec_combine)(uint32_t* x, const uint32_t* s, uint64_t n, const uint32_t* c0,
                                    const uint32_t* c1, const uint32_t* c2, uint64_t elements, const HostModulus& m,
                                    cudaStream_t stream);
-        // persistent batched transform with R = radix_bits register bits (2 or 3)
-        cudaError_t (*ntt_batched)(const BatchedParams& bp, int radix_bits, const HostModulus& m, unsigned grid,
-                                   size_t smem, cudaStream_t stream);
-        int (*ntt_batched_blocks_per_sm)(int radix_bits, size_t smem);
-        int radix_bits;
+        // persistent batched transform over pair passes planned for `block` threads
+        cudaError_t (*ntt_batched)(const BatchedParams& bp, bool inverse, const HostModulus& m, unsigned grid,
+                                   unsigned block, size_t smem, cudaStream_t stream);
+        int (*ntt_batched_blocks_per_sm)(bool inverse, unsigned block, size_t smem);
         cudaError_t (*lhe_combine_pair)(uint32_t* c0, uint32_t* c1, const uint32_t* ka, const uint32_t* kb,
                                         uint64_t n, const uint32_t* stacked, uint64_t elements,
                                         const HostModulus& m, cudaStream_t stream);
@@ -99,6 +97,9 @@ namespace hmpc_gb300
         // (for the tensor-core engine, whose first group reads memory)
         cudaError_t (*uniform_pairs)(uint32_t* out, uint32_t log_n, uint64_t elements, const RngKey& rng,
                                      int words, uint32_t top_mask, const HostModulus& m, cudaStream_t stream);
+        // one pass of the one-butterfly-per-thread transform (pair.cuh)
+        cudaError_t (*ntt_pair)(const PairPassParams& p, int kind, int nw, bool inverse, const HostModulus& m,
+                                unsigned grid, unsigned block, size_t smem, cudaStream_t stream);
     };
 
     // sizes of one tensor-core group kernel instantiation (TcShape)

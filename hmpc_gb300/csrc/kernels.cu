@@ -7,6 +7,7 @@
 #include "elementwise.cuh"
 #include "linalg.cuh"
 #include "ntt.cuh"
+#include "pair.cuh"
 
 #ifndef HMPC_L
 #error "compile with -DHMPC_L=<limbs>"
@@ -20,7 +21,6 @@ namespace hmpc_gb300
     namespace
     {
         constexpr int L = HMPC_L;
-        constexpr int R = 3;  // 8 elements per thread in the NTT passes
 
         Modulus<L> device_modulus(const HostModulus& h)
         {
@@ -51,21 +51,10 @@ namespace hmpc_gb300
             return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(g, 152ull * 64ull)));
         }
 
-        template<int Kind, int NW, int RB>
-        cudaError_t launch_pass(const NttPassParams& p, const Modulus<L>& m, unsigned grid, unsigned block,
+        template<int Kind, int NW, bool Inverse>
+        cudaError_t launch_pair(const PairPassParams& p, const Modulus<L>& m, unsigned grid, unsigned block,
                                 size_t smem, cudaStream_t stream)
         {
-            auto kernel = ntt_pass_kernel<L, RB, Kind, NW>;
-            static bool configured = false;
-            if (!configured)
-            {
-                cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-                if (e != cudaSuccess)
-                {
-                    return e;
-                }
-                configured = true;
-            }
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3(grid);
             cfg.blockDim = dim3(block);
@@ -76,53 +65,39 @@ namespace hmpc_gb300
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
             cfg.numAttrs = p.dependent ? 1u : 0u;
-            return cudaLaunchKernelEx(&cfg, kernel, p, m);
+            return cudaLaunchKernelEx(&cfg, ntt_pair_kernel<L, Kind, NW, Inverse>, p, m);
         }
 
-        template<int RB>
-        cudaError_t ntt_pass_radix(const NttPassParams& p, int kind, int nw, const Modulus<L>& m, unsigned grid,
-                                   unsigned block, size_t smem, cudaStream_t stream)
+        cudaError_t ntt_pair(const PairPassParams& p, int kind, int nw, bool inverse, const HostModulus& h,
+                             unsigned grid, unsigned block, size_t smem, cudaStream_t stream)
         {
+            const Modulus<L> m = device_modulus(h);
+            if (inverse)
+            {
+                return launch_pair<producer_tensor, 1, true>(p, m, grid, block, smem, stream);
+            }
             if (kind == producer_tensor)
             {
-                return launch_pass<producer_tensor, 1, RB>(p, m, grid, block, smem, stream);
+                return launch_pair<producer_tensor, 1, false>(p, m, grid, block, smem, stream);
             }
             if (kind == producer_cbd)
             {
                 switch (nw)
                 {
-                case 1: return launch_pass<producer_cbd, 1, RB>(p, m, grid, block, smem, stream);
-                case 2: return launch_pass<producer_cbd, 2, RB>(p, m, grid, block, smem, stream);
-                case 3: return launch_pass<producer_cbd, 3, RB>(p, m, grid, block, smem, stream);
-                case 4: return launch_pass<producer_cbd, 4, RB>(p, m, grid, block, smem, stream);
+                case 1: return launch_pair<producer_cbd, 1, false>(p, m, grid, block, smem, stream);
+                case 2: return launch_pair<producer_cbd, 2, false>(p, m, grid, block, smem, stream);
+                case 3: return launch_pair<producer_cbd, 3, false>(p, m, grid, block, smem, stream);
+                case 4: return launch_pair<producer_cbd, 4, false>(p, m, grid, block, smem, stream);
                 default: return cudaErrorInvalidValue;
                 }
             }
-            if (kind == producer_uniform)
+            if (kind == producer_uniform && nw == L + 2)
             {
-                if (nw == L + 2)
-                {
-                    return launch_pass<producer_uniform, L + 2, RB>(p, m, grid, block, smem, stream);
-                }
-                if (nw == L + 3)
-                {
-                    return launch_pass<producer_uniform, L + 3, RB>(p, m, grid, block, smem, stream);
-                }
+                return launch_pair<producer_uniform, L + 2, false>(p, m, grid, block, smem, stream);
             }
-            return cudaErrorInvalidValue;
-        }
-
-        cudaError_t ntt_pass(const NttPassParams& p, int kind, int nw, int radix_bits, const HostModulus& h,
-                             unsigned grid, unsigned block, size_t smem, cudaStream_t stream)
-        {
-            const Modulus<L> m = device_modulus(h);
-            if (radix_bits == 2)
+            if (kind == producer_uniform && nw == L + 3)
             {
-                return ntt_pass_radix<2>(p, kind, nw, m, grid, block, smem, stream);
-            }
-            if (radix_bits == 3)
-            {
-                return ntt_pass_radix<3>(p, kind, nw, m, grid, block, smem, stream);
+                return launch_pair<producer_uniform, L + 3, false>(p, m, grid, block, smem, stream);
             }
             return cudaErrorInvalidValue;
         }
@@ -343,45 +318,29 @@ namespace hmpc_gb300
             return cudaGetLastError();
         }
 
-        template<int RB>
-        cudaError_t launch_batched(const BatchedParams& bp, const Modulus<L>& m, unsigned grid, size_t smem,
-                                   cudaStream_t stream)
-        {
-            // the shared-memory attribute is set by ntt_batched_blocks_per_sm, which
-            // the batch planner calls before it captures this launch
-            ntt_batched_kernel<L, RB><<<grid, 256, smem, stream>>>(bp, m);
-            return cudaGetLastError();
-        }
-
-        cudaError_t ntt_batched(const BatchedParams& bp, int radix_bits, const HostModulus& h, unsigned grid,
-                                size_t smem, cudaStream_t stream)
+        cudaError_t ntt_batched(const BatchedParams& bp, bool inverse, const HostModulus& h, unsigned grid,
+                                unsigned block, size_t smem, cudaStream_t stream)
         {
             const Modulus<L> m = device_modulus(h);
-            if (radix_bits == 2)
+            if (inverse)
             {
-                return launch_batched<2>(bp, m, grid, smem, stream);
-            }
-            if (radix_bits == 3)
-            {
-                return launch_batched<3>(bp, m, grid, smem, stream);
-            }
-            return cudaErrorInvalidValue;
-        }
-
-        int ntt_batched_blocks_per_sm(int radix_bits, size_t smem)
-        {
-            int blocks = 0;
-            cudaError_t e;
-            if (radix_bits == 2)
-            {
-                cudaFuncSetAttribute(ntt_batched_kernel<L, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, ntt_batched_kernel<L, 2>, 256, smem);
+                ntt_batched_kernel<L, true><<<grid, block, smem, stream>>>(bp, m);
             }
             else
             {
-                cudaFuncSetAttribute(ntt_batched_kernel<L, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, ntt_batched_kernel<L, 3>, 256, smem);
+                ntt_batched_kernel<L, false><<<grid, block, smem, stream>>>(bp, m);
             }
+            return cudaGetLastError();
+        }
+
+        int ntt_batched_blocks_per_sm(bool inverse, unsigned block, size_t smem)
+        {
+            int blocks = 0;
+            const cudaError_t e =
+                inverse ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, ntt_batched_kernel<L, true>,
+                                                                        static_cast<int>(block), smem)
+                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, ntt_batched_kernel<L, false>,
+                                                                        static_cast<int>(block), smem);
             return e == cudaSuccess ? blocks : 0;
         }
 
@@ -473,10 +432,10 @@ namespace hmpc_gb300
             return cudaGetLastError();
         }
 
-        const KernelTable table = {ntt_pass, fma, binary, lhe_combine, uniform, cbd, to_montgomery,
+        const KernelTable table = {fma, binary, lhe_combine, uniform, cbd, to_montgomery,
                                    from_montgomery, cast, plain_stage, ct_mul, dec_combine, ntt_batched,
-                                   ntt_batched_blocks_per_sm, R, lhe_combine_pair, matvec, matvec_monomial,
-                                   reduce, equal, ntt_cluster, uniform_pairs};
+                                   ntt_batched_blocks_per_sm, lhe_combine_pair, matvec, matvec_monomial,
+                                   reduce, equal, ntt_cluster, uniform_pairs, ntt_pair};
     }
 
     const KernelTable* HMPC_CAT(kernel_table_, HMPC_L)()

@@ -1,0 +1,315 @@
+// Negacyclic NTT / INTT passes with one butterfly per thread and stage.
+//
+// Semantics are those of hmpc's stage-per-kernel transform
+// (hmpc/expr/number_theoretic_transform.hpp:90-197,262-549):
+//   forward stage s: length = 2^s, the lower element idx of a pair takes
+//     psi = T[2^s + (idx >> (n - s))]; v *= psi; (u+v, u-v)
+//   inverse stage s: psi = T[N/2^(s+1) + (idx >> (s+1))]; (u+v, (u-v)*psi); the
+//     last stage multiplies u+v by T[0] = N^-1 and u-v by T[1]
+//
+// A pass covers w consecutive stages; the w element-index bits they touch are
+// the rows of a tile, 2^c consecutive lower indices its columns (coalescing).
+// A tile is 2^(w+c-1) threads, each holding the two elements of a butterfly.
+// Between stages a thread keeps one of its two elements and trades the other
+// with the thread whose index differs in one bit: by shuffles when that bit
+// lies in the warp, through shared memory otherwise.
+//
+// Bound by the wide multiply-adds of the butterflies' products where the
+// polynomials fill the SMs (256 of 2^15 at 8 limbs: 1154 us, 0.82 of the
+// product rate), by the latency of the stages where they do not.  One
+// butterfly per thread and one copy of the product's code in the stage loop:
+// holding 8 elements in registers and unrolling three stages of butterflies
+// touches shared memory a third as often, which the products hide anyway,
+// but left a small transform with a quarter of the warps and about 150 KB of
+// straight-line code to fetch.  Against that form, tuned: one polynomial of
+// 2^15 at 8 limbs 55.8 -> 15.0 us, 3 of 2^13 49.2 -> 12.7, 33 of 2^14 at 6
+// limbs 71 -> 54, 256 of 2^15 at 8 limbs 1334 -> 1154.
+#pragma once
+
+#include <cstdint>
+
+#include "chacha.cuh"
+#include "limbs.cuh"
+#include "ntt.cuh"
+
+namespace hmpc_gb300
+{
+    constexpr uint32_t pair_max_threads = 512;
+
+    struct PairPassParams
+    {
+        uint32_t* out;                 // limb-planar, `elements` entries per limb
+        const uint32_t* src;           // tensor producer input (nullptr: read out)
+        const uint32_t* twiddles;      // element-major [N][L]
+        const uint32_t* small_table;   // Montgomery forms of 0..64, element-major
+        uint64_t elements;             // batch * N
+        uint64_t tiles;                // batch * tiles per polynomial
+        uint32_t log_n;
+        uint32_t w, c;                 // stages of this pass, column bits
+        uint32_t row_shift;            // element bit of the lowest row bit
+        RngKey rng;
+        uint32_t vx2;                  // 2V for the CBD producer
+        uint32_t top_mask;             // uniform producer: mask of the top word
+        const uint32_t* poly_rng;      // per-polynomial RNG, see pair_generator
+        uint32_t rng_slot;
+        uint32_t dependent;            // host side: programmatic dependence on the pass before
+    };
+
+    // One pass over the tiles of block `block` of the pass's grid.  exchange
+    // holds [2][L][blockDim.x] words.  Wait: whether the input may still be
+    // being written by the kernel before this one in the stream.
+    template<int L, int Kind, int NW, bool Inverse, bool Wait>
+    __device__ __forceinline__ void ntt_pair_process(const PairPassParams& p, const Modulus<L>& m, uint64_t block,
+                                                     uint32_t* exchange)
+    {
+        const uint32_t t = threadIdx.x;
+        const uint32_t w = p.w, c = p.c;
+        const uint32_t pair_bits = w + c - 1;
+        const uint64_t tile = block * (blockDim.x >> pair_bits) + (t >> pair_bits);
+        const bool active = tile < p.tiles;
+        const uint32_t col = t & ((1u << c) - 1u);
+        const uint32_t r = (t >> c) & ((1u << (w - 1)) - 1u);  // the row bits but the pair's
+        const uint32_t tile_bits = p.log_n - w - c;
+        const uint64_t poly = tile >> tile_bits;
+        const uint32_t in_poly = static_cast<uint32_t>(tile) & ((1u << tile_bits) - 1u);
+        const uint32_t mid_bits = p.row_shift - c;
+        const uint32_t high = in_poly >> mid_bits;  // index bits above the rows
+        const uint32_t base = (high << (p.row_shift + w)) | ((in_poly & ((1u << mid_bits) - 1u)) << c) | col;
+        const uint64_t poly_base = poly << p.log_n;
+        // Stage j of the pass pairs row bit w-1-j (forward) or j (inverse).  The
+        // thread bits above that one stand for the row bits above it, one to
+        // one, so both the twiddle and the rows follow from r by shifts.
+        const uint32_t twiddle_high = (1u << (p.log_n - p.row_shift - w)) + high;
+        auto twiddle_index = [&](uint32_t j) {
+            return Inverse ? (twiddle_high << (w - 1 - j)) + (r >> j) : (twiddle_high << j) + (r >> (w - 1 - j));
+        };
+        uint32_t lo[L], hi[L], tw[L];
+        load_twiddle<L>(tw, p.twiddles, twiddle_index(0));
+        if constexpr (Wait)
+        {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
+        {
+            const uint32_t row = Inverse ? r << 1 : r;
+            const uint32_t idx = base | (row << p.row_shift);
+            const uint32_t step = 1u << (p.row_shift + (Inverse ? 0u : w - 1));
+            if constexpr (Kind != producer_tensor)
+            {
+                if (active)
+                {
+                    produce_pair<L, Kind, NW>(p, m, poly, idx, idx + step, lo, hi);
+                }
+                else
+                {
+                    set_zero<L>(lo);
+                    set_zero<L>(hi);
+                }
+            }
+            else
+            {
+                const uint32_t* in = (p.src ? p.src : p.out) + poly_base + idx;
+#pragma unroll
+                for (int j = 0; j < L; ++j)
+                {
+                    lo[j] = active ? in[static_cast<uint64_t>(j) * p.elements] : 0u;
+                    hi[j] = active ? in[static_cast<uint64_t>(j) * p.elements + step] : 0u;
+                }
+            }
+        }
+        uint32_t* buffer = exchange;
+        uint32_t* other = exchange + L * blockDim.x;
+#pragma unroll 1
+        for (uint32_t j = 0; j < w; ++j)
+        {
+            if (j > 0)
+            {
+                const uint32_t bit = c + (Inverse ? j - 1 : w - 1 - j);
+                const bool upper = (t >> bit) & 1u;
+                if (bit < 5)
+                {
+#pragma unroll
+                    for (int k = 0; k < L; ++k)
+                    {
+                        const uint32_t v = __shfl_xor_sync(0xffffffffu, upper ? lo[k] : hi[k], 1 << bit);
+                        lo[k] = upper ? v : lo[k];
+                        hi[k] = upper ? hi[k] : v;
+                    }
+                }
+                else
+                {
+#pragma unroll
+                    for (int k = 0; k < L; ++k)
+                    {
+                        buffer[k * blockDim.x + t] = upper ? lo[k] : hi[k];
+                    }
+                    __syncthreads();
+#pragma unroll
+                    for (int k = 0; k < L; ++k)
+                    {
+                        const uint32_t v = buffer[k * blockDim.x + (t ^ (1u << bit))];
+                        lo[k] = upper ? v : lo[k];
+                        hi[k] = upper ? hi[k] : v;
+                    }
+                    // the next exchange writes the other buffer: a thread gets
+                    // there only after this barrier's readers of it are done
+                    uint32_t* swap = buffer;
+                    buffer = other;
+                    other = swap;
+                }
+            }
+            uint32_t next[L];
+            load_twiddle<L>(next, p.twiddles, twiddle_index(j + 1 < w ? j + 1 : j));
+            if constexpr (!Inverse)
+            {
+                mont_mul<L>(hi, hi, tw, m);
+                uint32_t sum[L];
+                mod_add<L>(sum, lo, hi, m);
+                mod_sub<L>(hi, lo, hi, m);
+#pragma unroll
+                for (int k = 0; k < L; ++k)
+                {
+                    lo[k] = sum[k];
+                }
+            }
+            else
+            {
+                uint32_t sum[L];
+                mod_add<L>(sum, lo, hi, m);
+                mod_sub<L>(hi, lo, hi, m);
+#pragma unroll
+                for (int k = 0; k < L; ++k)
+                {
+                    lo[k] = sum[k];
+                }
+                if (p.row_shift + j == p.log_n - 1)
+                {
+                    // the transform's last stage: tw is T[1], and u + v takes T[0] = N^-1
+                    uint32_t scale[L];
+                    load_twiddle<L>(scale, p.twiddles, 0u);
+                    mont_mul<L>(lo, lo, scale, m);
+                }
+                mont_mul<L>(hi, hi, tw, m);
+            }
+#pragma unroll
+            for (int k = 0; k < L; ++k)
+            {
+                tw[k] = next[k];
+            }
+        }
+        if (active)
+        {
+            const uint32_t row = Inverse ? r : r << 1;
+            const uint32_t step = 1u << (p.row_shift + (Inverse ? w - 1 : 0u));
+            uint32_t* out = p.out + poly_base + (base | (row << p.row_shift));
+#pragma unroll
+            for (int j = 0; j < L; ++j)
+            {
+                out[static_cast<uint64_t>(j) * p.elements] = lo[j];
+                out[static_cast<uint64_t>(j) * p.elements + step] = hi[j];
+            }
+        }
+    }
+
+    template<int L, int Kind, int NW, bool Inverse>
+    __global__ void __launch_bounds__(pair_max_threads) ntt_pair_kernel(const PairPassParams p, const Modulus<L> m)
+    {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        extern __shared__ uint32_t exchange[];
+        ntt_pair_process<L, Kind, NW, Inverse, true>(p, m, blockIdx.x, exchange);
+    }
+
+    // ----------------------------------------------------------------------
+    // Persistent transform over a batch of polynomials of uneven degree.
+    // Work items are (pass of one polynomial, CTA tile group) in a list that
+    // holds every first-pass item before any later-pass item; CTAs take items
+    // in list order from an atomic counter.  An item of pass k of a
+    // polynomial waits until all earlier-pass items of that polynomial have
+    // signalled.  Every item it waits for was taken earlier by a running CTA
+    // that never waits on later items, so the waits end; they are still
+    // bounded, and a wait that runs out sets `error` and the kernel returns.
+    struct BatchedControl
+    {
+        uint32_t next;      // work counter
+        uint32_t error;     // nonzero: a wait ran out (value = item + 1)
+        uint32_t done;      // items finished
+        uint32_t pad;
+    };
+
+    struct BatchedParams
+    {
+        const PairPassParams* params;   // one per (polynomial, pass)
+        const uint32_t* item_param;     // item -> params index
+        const uint32_t* item_tile;      // item -> CTA tile group inside that pass
+        const uint32_t* item_wait;      // item -> signals needed before it may start (0: none)
+        const uint32_t* item_poly;      // item -> polynomial (counter index)
+        const uint32_t* item_signal;    // item -> 1 when it must signal its polynomial
+        uint32_t* counters;             // per polynomial
+        BatchedControl* control;
+        uint32_t items;
+        uint32_t spin_limit;            // polls of 64 ns before a wait gives up
+    };
+
+    __device__ __forceinline__ uint32_t load_acquire(const uint32_t* ptr)
+    {
+        uint32_t v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ptr) : "memory");
+        return v;
+    }
+
+    template<int L, bool Inverse>
+    __global__ void __launch_bounds__(pair_max_threads) ntt_batched_kernel(const BatchedParams bp, const Modulus<L> m)
+    {
+        extern __shared__ uint32_t exchange[];
+        __shared__ uint32_t item_s;
+        __shared__ uint32_t abort_s;
+        for (;;)
+        {
+            if (threadIdx.x == 0)
+            {
+                uint32_t item = atomicAdd(&bp.control->next, 1u);
+                uint32_t abort = 0;
+                if (item < bp.items)
+                {
+                    const uint32_t need = bp.item_wait[item];
+                    if (need)
+                    {
+                        const uint32_t* counter = bp.counters + bp.item_poly[item];
+                        uint32_t polls = 0;
+                        while (load_acquire(counter) < need)
+                        {
+                            if (++polls > bp.spin_limit || load_acquire(&bp.control->error))
+                            {
+                                atomicCAS(&bp.control->error, 0u, item + 1u);
+                                abort = 1;
+                                break;
+                            }
+                            __nanosleep(64);
+                        }
+                    }
+                }
+                item_s = item;
+                abort_s = abort;
+            }
+            __syncthreads();
+            const uint32_t item = item_s;
+            const uint32_t abort = abort_s;
+            __syncthreads();
+            if (item >= bp.items || abort)
+            {
+                return;
+            }
+            const PairPassParams& p = bp.params[bp.item_param[item]];
+            ntt_pair_process<L, producer_tensor, 1, Inverse, false>(p, m, bp.item_tile[item], exchange);
+            __syncthreads();
+            if (threadIdx.x == 0)
+            {
+                if (bp.item_signal[item])
+                {
+                    __threadfence();
+                    atomicAdd(bp.counters + bp.item_poly[item], 1u);
+                }
+                atomicAdd(&bp.control->done, 1u);
+            }
+        }
+    }
+}

@@ -9,7 +9,7 @@
 
 #include "chacha.cuh"
 #include "limbs.cuh"
-#include "ntt.cuh"
+#include "pair.cuh"
 
 namespace hmpc_gb300
 {
@@ -49,7 +49,7 @@ namespace hmpc_gb300
             uint32_t u[L], v[L], t[L];
             if (Kind != producer_tensor && s == 0)
             {
-                NttPassParams q{};
+                PairPassParams q{};
                 q.log_n = p.log_n;
                 q.rng = p.rng;
                 q.vx2 = p.vx2;

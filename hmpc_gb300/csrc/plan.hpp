@@ -1,173 +1,84 @@
-// Pass planner for the tiled transform (see ntt.cuh): splits the log2(N)
-// stages into shared-memory passes and each pass into register groups.
+// Pass planner of the one-butterfly-per-thread transform (pair.cuh).
 #pragma once
 
 #include <algorithm>
 #include <cstdint>
 #include <vector>
 
-#include "ntt.cuh"
+#include "pair.cuh"
 
 namespace hmpc_gb300
 {
-    struct PassPlan
-    {
-        NttPassParams params;
-        unsigned grid = 0;
-        unsigned block = 0;
-        size_t smem = 0;
-    };
-
-    struct PlanOptions
-    {
-        int max_local_bits = 0;   // 0: derived from the shared-memory budget
-        int col_bits = 4;         // preferred coalescing width (2^c consecutive elements)
-        int smem_budget = 112 * 1024;
-        bool spread_small_batches = true;  // shrink CTA tiles to fill the GPU when the batch is small
-    };
-
-    inline uint32_t smem_words(uint32_t local_count)
-    {
-        return local_count + (local_count >> 5);
-    }
-
-    inline int local_bits_for(int limbs, const PlanOptions& o)
-    {
-        if (o.max_local_bits)
-        {
-            return o.max_local_bits;
-        }
-        int b = 13;
-        while (b > 4 && static_cast<uint64_t>(limbs) * 4u * smem_words(1u << b) > static_cast<uint64_t>(o.smem_budget))
-        {
-            --b;
-        }
-        return b;
-    }
-
     struct BitRange
     {
         int lo, hi, c;
     };
 
-    // Bit ranges in forward-stage order (top bits first).
-    inline std::vector<BitRange> plan_ranges(int log_n, int b, int col_pref)
+    struct PairPlan
     {
-        std::vector<BitRange> r;
+        PairPassParams params;
+        unsigned grid = 0;
+        unsigned block = 0;
+        size_t smem = 0;
+    };
+
+    // Passes of the one-butterfly-per-thread transform (pair.cuh): the low
+    // `tile_bits` index bits are one pass over contiguous elements, the bits
+    // above them column passes of at least 2^col_bits consecutive elements.
+    // tile_bits 0: the shape by the rule below, measured over 1 to 256
+    // polynomials of 2^12..2^20, 2 to 8 limbs, all shapes of tile bits 6..10 and
+    // column bits 2..5.  Fewest passes first: 2^13 takes two at tile bits 8,
+    // 2^15 at 9, 2^16 at 9 with column bits 2 (127 against 135 us with a third
+    // pass, 32 polynomials at 4 limbs), 2^17 at 10.  Above that the shapes are
+    // within a few per cent of one another, except where there is at most one
+    // warp per scheduler: then the smaller tile spreads it over twice the SMs
+    // (one polynomial of 2^15 at 8 limbs: 15.0 us in three passes at tile bits
+    // 8, 18.5 in two at 9; two polynomials: 24.6 and 18.4).
+    // block: threads of every pass's blocks, at least 2^(tile_bits - 1) (0: by
+    // the size).
+    inline std::vector<PairPlan> plan_pairs(int limbs, int log_n, uint64_t batch, bool inverse, int tile_bits,
+                                            int col_bits, unsigned block = 0)
+    {
+        if (tile_bits == 0)
+        {
+            // one warp per scheduler or less: small tiles spread over the SMs
+            const bool sparse = (batch << (log_n - 1)) <= 152ull * 128;
+            tile_bits = log_n <= 13 || (sparse && log_n <= 15) ? 8 : log_n <= 16 ? 9 : 10;
+            col_bits = log_n == 16 ? 2 : 3;
+        }
+        tile_bits = std::min(tile_bits, 10);
+        const int contiguous = std::min(log_n, tile_bits);
+        const int rest = log_n - contiguous;
+        const int widest = std::max(1, tile_bits - col_bits);
+        const int columns = (rest + widest - 1) / widest;
+        std::vector<BitRange> ranges;  // forward order: top bits first
         int hi = log_n;
-        while (hi > b)
+        for (int i = 0; i < columns; ++i)
         {
-            int w = std::max(1, b - col_pref);
-            if (hi - w < 1)
-            {
-                w = hi - 1;
-            }
-            // keep the final contiguous pass within the budget: never leave more
-            // than b bits below unless another column pass follows
-            const int lo = hi - w;
-            const int c = std::min(std::min(b - w, lo), 5);
-            r.push_back({lo, hi, c});
-            hi = lo;
+            const int w = rest / columns + (i < rest % columns ? 1 : 0);
+            ranges.push_back({hi - w, hi, std::max(0, std::min({tile_bits - w, hi - w, 5}))});
+            hi -= w;
         }
-        r.push_back({0, hi, 0});
-        return r;
-    }
-
-    // every pass must hold at least one full register group inside a tile
-    // (c + w >= R); shrink the column pass above a too-narrow final pass
-    inline void keep_register_groups(std::vector<BitRange>& r, int R, int b)
-    {
-        if (r.size() >= 2 && r.back().hi < R)
-        {
-            BitRange& prev = r[r.size() - 2];
-            const int grow = R - r.back().hi;
-            prev.lo += grow;
-            prev.c = std::min(std::min(b - (prev.hi - prev.lo), prev.lo), 5);
-            r.back().hi += grow;
-        }
-    }
-
-    inline std::vector<PassPlan> plan_transform(int limbs, int log_n, uint64_t batch, bool inverse, int R,
-                                                const PlanOptions& o = {})
-    {
-        const int b = local_bits_for(limbs, o);
-        std::vector<BitRange> ranges = plan_ranges(log_n, b, o.col_bits);
-        keep_register_groups(ranges, R, b);
+        ranges.push_back({0, contiguous, 0});
         if (inverse)
         {
             std::reverse(ranges.begin(), ranges.end());
         }
-        std::vector<PassPlan> out;
+        std::vector<PairPlan> out;
         for (const BitRange& rg : ranges)
         {
-            PassPlan pp{};
-            NttPassParams& p = pp.params;
-            const int w = rg.hi - rg.lo;
-            const int c = rg.c;
+            PairPlan pp{};
+            PairPassParams& p = pp.params;
             p.log_n = static_cast<uint32_t>(log_n);
-            p.inverse = inverse ? 1u : 0u;
-            if (inverse)
-            {
-                p.s0 = static_cast<uint32_t>(rg.lo);
-                p.s1 = static_cast<uint32_t>(rg.hi);
-            }
-            else
-            {
-                p.s0 = static_cast<uint32_t>(log_n - rg.hi);
-                p.s1 = static_cast<uint32_t>(log_n - rg.lo);
-            }
+            p.w = static_cast<uint32_t>(rg.hi - rg.lo);
+            p.c = static_cast<uint32_t>(rg.c);
             p.row_shift = static_cast<uint32_t>(rg.lo);
-            p.col_bits = static_cast<uint32_t>(c);
-            const uint64_t tiles_per_poly = 1ull << (log_n - w - c);
-            p.tiles = batch * tiles_per_poly;
-            int tile_bits = std::max(0, b - w - c);
-            if (!o.spread_small_batches)
-            {
-                // whole CTA groups inside one polynomial
-                tile_bits = std::min(tile_bits, log_n - w - c);
-            }
-            tile_bits = std::max(tile_bits, R - w - c);
-            // keep at least ~2 CTAs per SM when the batch is small, as long as a
-            // CTA still holds a full register block per thread
-            while (o.spread_small_batches && tile_bits > 0 && tile_bits + w + c > R + 5 &&
-                   ((p.tiles + (1ull << tile_bits) - 1) >> tile_bits) < 304)
-            {
-                --tile_bits;
-            }
-            p.tile_bits = static_cast<uint32_t>(tile_bits);
-            p.local_bits = static_cast<uint32_t>(tile_bits + w + c);
-            // register groups
-            int g = 0;
-            for (int s = static_cast<int>(p.s0); s < static_cast<int>(p.s1); s += R, ++g)
-            {
-                NttGroup& grp = p.groups[g];
-                grp.stage = static_cast<uint32_t>(s);
-                grp.count = static_cast<uint32_t>(std::min(R, static_cast<int>(p.s1) - s));
-                uint32_t used = 0;
-                for (int k = 0; k < static_cast<int>(grp.count); ++k)
-                {
-                    const int stage = s + k;
-                    const int bit = inverse ? stage : (log_n - 1 - stage);
-                    const int local = c + (bit - rg.lo);
-                    grp.reg_pos[k] = static_cast<uint32_t>(local);
-                    used |= 1u << local;
-                }
-                int next = 0;
-                for (int k = static_cast<int>(grp.count); k < R; ++k)
-                {
-                    while (used & (1u << next))
-                    {
-                        ++next;
-                    }
-                    grp.reg_pos[k] = static_cast<uint32_t>(next);
-                    used |= 1u << next;
-                }
-                grp.rest_mask = ((1u << p.local_bits) - 1u) & ~used;
-            }
-            p.num_groups = static_cast<uint32_t>(g);
-            pp.grid = static_cast<unsigned>((p.tiles + (1ull << tile_bits) - 1) >> tile_bits);
-            pp.block = static_cast<unsigned>(std::min<uint32_t>(256u, 1u << (p.local_bits - R)));
-            pp.smem = static_cast<size_t>(limbs) * 4u * smem_words(1u << p.local_bits);
+            p.tiles = batch << (log_n - static_cast<int>(p.w + p.c));
+            const unsigned tile_threads = 1u << (p.w + p.c - 1);
+            pp.block = block ? block : std::max(tile_threads, p.tiles * tile_threads >= 152ull * 256 ? 128u : 32u);
+            const uint64_t per_block = pp.block / tile_threads;
+            pp.grid = static_cast<unsigned>((p.tiles + per_block - 1) / per_block);
+            pp.smem = 2ull * static_cast<size_t>(limbs) * pp.block * sizeof(uint32_t);
             out.push_back(pp);
         }
         return out;

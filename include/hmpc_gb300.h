@@ -98,9 +98,10 @@ int hmpc_modulus_prepare(hmpc_modulus* mod, uint64_t n);
  * L words (hmpc/ints/num/theory/root_of_unity.hpp:20-54). */
 int hmpc_modulus_root(hmpc_modulus* mod, uint64_t n, int inverse, uint32_t* root);
 /* Tile shape of the transforms of degree n over `batch` polynomials in one
- * direction: register radix bits (2 or 3: 4 or 8 elements per thread), tile
- * bits (log2 elements a CTA stages; 0 = by shared-memory budget) and column
- * bits (coalescing width) -- or radix bits 0: the tensor-core engine (exact
+ * direction: radix bits 2 or 3 (both: the CUDA-core tiles, one butterfly per
+ * thread), tile bits (log2 elements of a tile, at most 10 are used; 0 = tile
+ * and column bits by a rule on the sizes) and column bits (consecutive
+ * elements of a tile's rows) -- or radix bits 0: the tensor-core engine (exact
  * fp16 MMAs over 8-bit digits, moduli of 2 to 8 limbs below
  * 0.996 * 2^(32L); tensor, CBD(V) and forward uniform producers, the
  * uniform draws written to the output by one launch before the groups run in
