@@ -75,6 +75,12 @@ namespace hmpc_gb300::detail
         return HMPC_OK;
     }
 
+    bool capturing(const hmpc_context* ctx)
+    {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        return cudaStreamIsCapturing(ctx->stream, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+    }
+
     int run_transform(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, bool inverse, int kind,
                       uint32_t vx2, uint32_t security, const uint32_t* src, uint32_t* out, const uint32_t* poly_rng,
                       uint32_t rng_slot, bool cuda_cores_only)
@@ -205,15 +211,13 @@ namespace hmpc_gb300::detail
         // 20.9 -> 14.9 us (one polynomial of 2^15 at 8 limbs), 18.8 -> 16.2 us
         // (12 of 2^13 at 6), 297.3 -> 295.2 us (64 of 2^15 at 8): never slower.
         // Ordinary launches while the stream is being captured.
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        const bool capturing =
-            cudaStreamIsCapturing(ctx->stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone;
+        const bool dependent = !capturing(ctx);
         const std::vector<PairPlan> plan = plan_pairs(L, log_n, batch, inverse, choice.local_bits, choice.col_bits);
         for (size_t i = 0; i < plan.size(); ++i)
         {
             PairPassParams p = plan[i].params;
-            p.dependent = capturing ? 0u : 1u;
-            p.out = out;
+            p.dependent = dependent ? 1u : 0u;
+            p.out[0] = out;
             p.src = i == 0 ? src : nullptr;
             p.twiddles = inverse ? t->inverse : t->forward;
             p.small_table = mod->small_table;
@@ -337,6 +341,140 @@ namespace hmpc_gb300::detail
             rc = run_transform(ctx, p, n, batch, false, producer_tensor, 0, 0, out, out);
         }
         return rc;
+    }
+
+    bool parts_applicable(const hmpc_modulus* q, const hmpc_modulus* p)
+    {
+        // p times a sample plus a lifted residue stays below 2^70 < Q
+        return p->c.limbs <= 2 && q->c.bits >= 72;
+    }
+
+    // Forward transforms of `count` parts of `batch` polynomials as one run of
+    // passes: part i is drawn as kinds[i] with nonce ctx->nonce + slots[i] * n *
+    // batch (or from poly_rng's descriptors with that slot) and goes to out[i].
+    int run_parts(hmpc_context* ctx, hmpc_modulus* q, const hmpc_modulus* p, uint64_t n, uint64_t batch, int count,
+                  const uint32_t* kinds, const uint32_t* slots, uint32_t* const* out, const uint32_t* msg,
+                  const uint32_t* poly_rng)
+    {
+        Tables* t = nullptr;
+        if (int rc = q->prepare(n, &t))
+        {
+            return rc;
+        }
+        const std::vector<PairPlan> plan = plan_pairs(q->c.limbs, __builtin_ctzll(n), batch * count, false, 0, 0);
+        const bool dependent = !capturing(ctx);
+        for (size_t i = 0; i < plan.size(); ++i)
+        {
+            PairPassParams pp = plan[i].params;
+            pp.part_polys = batch;
+            pp.elements = n * batch;
+            pp.twiddles = t->forward;
+            pp.small_table = q->small_table;
+            pp.rng = ctx->rng();
+            pp.poly_rng = poly_rng;
+            pp.dependent = dependent ? 1u : 0u;
+            for (int j = 0; j < count; ++j)
+            {
+                pp.out[j] = out[j];
+                pp.parts.kind[j] = kinds[j];
+                std::copy(ctx->nonce, ctx->nonce + 3, pp.parts.nonce[j]);
+                nonce_add(pp.parts.nonce[j], slots[j] * n * batch);
+            }
+            pp.parts.msg = msg;
+            pp.parts.msg_limbs = static_cast<uint32_t>(p->c.limbs);
+            for (int j = 0; j < p->c.limbs; ++j)
+            {
+                pp.parts.pq[j] = p->h.q[j];
+                pp.parts.phalf[j] = p->h.half[j];
+            }
+            pp.parts.pninv = p->h.ninv;
+            std::copy(q->h.r2, q->h.r2 + q->c.limbs, pp.parts.r2);
+            cudaError_t e = q->kt->ntt_pair(pp, i == 0 ? producer_parts : producer_tensor, 1, false, q->h,
+                                            plan[i].grid, plan[i].block, plan[i].smem, ctx->stream);
+            if (e != cudaSuccess)
+            {
+                return cuda_fail(e, "launching NTT pass");
+            }
+            ++ctx->launches;
+        }
+        return HMPC_OK;
+    }
+
+    int encrypt_cuda_cores(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n, uint64_t batch,
+                           const uint32_t* key_a, const uint32_t* key_b, const uint32_t* coefficients, uint32_t* c0,
+                           uint32_t* c1, uint32_t* workspace, const uint32_t* poly_rng, bool cuda_cores_only)
+    {
+        const uint64_t elements = n * batch;
+        const uint64_t poly_words = elements * static_cast<uint64_t>(q->c.limbs);
+        uint32_t* u = workspace;
+        uint32_t* v = u + poly_words;
+        uint32_t* msg = v + poly_words;
+        if (parts_applicable(q, p))
+        {
+            // linearity of the NTT: p*NTT(v) + NTT(lift(m)) = NTT(p*v + lift(m))
+            // and p*NTT(w) = NTT(p*w), so three transforms run as one and one
+            // kernel writes both halves.  Draws in the reference's order u, v, w
+            // (expr/cache.hpp:226-271).
+            const uint32_t kinds[3] = {part_ternary, part_scaled_message, part_scaled};
+            const uint32_t slots[3] = {0, 1, 2};
+            uint32_t* const outs[3] = {u, v, msg};
+            if (int rc = run_parts(ctx, q, p, n, batch, 3, kinds, slots, outs, coefficients, poly_rng))
+            {
+                return rc;
+            }
+            cudaError_t e = q->kt->lhe_combine_pair(c0, c1, key_a, key_b, n, u, v, msg, elements, elements,
+                                                    !capturing(ctx), q->h, ctx->stream);
+            if (e != cudaSuccess)
+            {
+                return cuda_fail(e, "launching combine");
+            }
+            ++ctx->launches;
+            if (!poly_rng)
+            {
+                nonce_add(ctx->nonce, 3 * elements);
+            }
+            return HMPC_OK;
+        }
+        // the reference's plan: NTT(u), NTT(v), NTT_q(msg), c0, NTT(w), c1
+        int rc = run_transform(ctx, q, n, batch, false, producer_cbd, 1, 0, nullptr, u, poly_rng, 0, cuda_cores_only);
+        if (!rc)
+        {
+            rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v, poly_rng, 1, cuda_cores_only);
+        }
+        if (rc)
+        {
+            return rc;
+        }
+        cudaError_t e = q->kt->cast(msg, coefficients, elements, make_cast(q, p), q->h, ctx->stream);
+        if (e != cudaSuccess)
+        {
+            return cuda_fail(e, "launching cast");
+        }
+        ++ctx->launches;
+        if ((rc = run_transform(ctx, q, n, batch, false, producer_tensor, 0, 0, msg, msg, nullptr, 0,
+                                cuda_cores_only)))
+        {
+            return rc;
+        }
+        const host::words pm = host::to_mont(q->c, p->c.q);
+        if ((e = q->kt->lhe_combine(c0, key_a, n, u, v, msg, elements, pm.data(), q->h, ctx->stream)) != cudaSuccess)
+        {
+            return cuda_fail(e, "launching combine");
+        }
+        ++ctx->launches;
+        // w reuses v's buffer
+        if ((rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v, poly_rng, 2,
+                                cuda_cores_only)))
+        {
+            return rc;
+        }
+        if ((e = q->kt->lhe_combine(c1, key_b, n, u, v, nullptr, elements, pm.data(), q->h, ctx->stream)) !=
+            cudaSuccess)
+        {
+            return cuda_fail(e, "launching combine");
+        }
+        ++ctx->launches;
+        return HMPC_OK;
     }
 
     // one launch per stage over global memory (plain.cuh)
@@ -484,19 +622,6 @@ int hmpc_context_destroy(hmpc_context* ctx)
     cudaFree(ctx->workspace);
     cudaFree(ctx->tc_workspace);
     cudaFree(ctx->tc_error);
-    if (ctx->aux_stream)
-    {
-        cudaStreamSynchronize(ctx->aux_stream);
-        cudaStreamDestroy(ctx->aux_stream);
-    }
-    if (ctx->fork_event)
-    {
-        cudaEventDestroy(ctx->fork_event);
-    }
-    if (ctx->join_event)
-    {
-        cudaEventDestroy(ctx->join_event);
-    }
     delete ctx;
     return HMPC_OK;
 }
@@ -1169,10 +1294,16 @@ int hmpc_lhe_enc(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n
     {
         return fail(HMPC_ERROR_OUT_OF_MEMORY, "allocating the encryption workspace");
     }
-    uint32_t* u = ws;
-    uint32_t* v = ws + poly_words;
-    uint32_t* msg = ws + 2 * poly_words;
     uint32_t* coeff = ws + 3 * poly_words;
+    const uint32_t* coefficients = plaintext;
+    if (plaintext_ntt)
+    {
+        if (int rc = run_transform(ctx, p, n, batch, true, producer_tensor, 0, 0, plaintext, coeff))
+        {
+            return rc;
+        }
+        coefficients = coeff;
+    }
     const int tc_splits = tc_plan_splits(q, n, batch);
     if (tc_splits && n >= 16 && tc_supported(q) && p->c.limbs <= 2)
     {
@@ -1185,13 +1316,6 @@ int hmpc_lhe_enc(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n
         // once and writes c0 and c1; every result is the reduced
         // representative, so the ciphertext is the reference's bit for bit.  RNG order as the
         // reference's plan: u, v, w (expr/cache.hpp:226-271).
-        int rc = HMPC_OK;
-        const uint32_t* coefficients = plaintext;
-        if (plaintext_ntt)
-        {
-            rc = run_transform(ctx, p, n, batch, true, producer_tensor, 0, 0, plaintext, coeff);
-            coefficients = coeff;
-        }
         const TcSmallInput with_msg{coefficients, p};
         const TcSmallInput no_msg{nullptr, p};
         TcStackPart parts[3];
@@ -1201,13 +1325,12 @@ int hmpc_lhe_enc(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n
         parts[2].vx2 = 20;
         parts[2].small = &no_msg;
         uint32_t* stacked = ws;  // [L][3 * elements]: u | p*v + lift(m) | p*w, in NTT form
+        int rc = run_tc_stacked(ctx, q, n, batch, parts, 3, stacked, tc_splits);
         if (!rc)
         {
-            rc = run_tc_stacked(ctx, q, n, batch, parts, 3, stacked, tc_splits);
-        }
-        if (!rc)
-        {
-            cudaError_t e = q->kt->lhe_combine_pair(c0, c1, key_a, key_b, n, stacked, elements, q->h, ctx->stream);
+            cudaError_t e = q->kt->lhe_combine_pair(c0, c1, key_a, key_b, n, stacked, stacked + elements,
+                                                    stacked + 2 * elements, 3 * elements, elements, !capturing(ctx),
+                                                    q->h, ctx->stream);
             if (e != cudaSuccess)
             {
                 return cuda_fail(e, "launching combine");
@@ -1216,50 +1339,7 @@ int hmpc_lhe_enc(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n
         }
         return rc;
     }
-    // the execution order of the reference's plan: NTT(u), NTT(v),
-    // [INTT_p(x)], NTT_q(msg), c0, NTT(w), c1 (expr/cache.hpp:226-271)
-    int rc = run_transform(ctx, q, n, batch, false, producer_cbd, 1, 0, nullptr, u);
-    if (!rc)
-    {
-        rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v);
-    }
-    const uint32_t* coefficients = plaintext;
-    if (!rc && plaintext_ntt)
-    {
-        rc = run_transform(ctx, p, n, batch, true, producer_tensor, 0, 0, plaintext, coeff);
-        coefficients = coeff;
-    }
-    if (!rc)
-    {
-        cudaError_t e = q->kt->cast(msg, coefficients, elements, make_cast(q, p), q->h, ctx->stream);
-        if (e != cudaSuccess)
-        {
-            return cuda_fail(e, "launching cast");
-        }
-        ++ctx->launches;
-        rc = run_transform(ctx, q, n, batch, false, producer_tensor, 0, 0, msg, msg);
-    }
-    const host::words pm = host::to_mont(q->c, p->c.q);
-    if (!rc)
-    {
-        cudaError_t e = q->kt->lhe_combine(c0, key_a, n, u, v, msg, elements, pm.data(), q->h, ctx->stream);
-        if (e != cudaSuccess)
-        {
-            return cuda_fail(e, "launching combine");
-        }
-        ++ctx->launches;
-        rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v);  // w reuses v's buffer
-    }
-    if (!rc)
-    {
-        cudaError_t e = q->kt->lhe_combine(c1, key_b, n, u, v, nullptr, elements, pm.data(), q->h, ctx->stream);
-        if (e != cudaSuccess)
-        {
-            return cuda_fail(e, "launching combine");
-        }
-        ++ctx->launches;
-    }
-    return rc;
+    return encrypt_cuda_cores(ctx, q, p, n, batch, key_a, key_b, coefficients, c0, c1, ws, nullptr, false);
 }
 
 int hmpc_lhe_dec(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n, uint64_t batch,
@@ -1336,42 +1416,38 @@ int hmpc_lhe_keygen(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_
     {
         return fail(HMPC_ERROR_OUT_OF_MEMORY, "allocating the key workspace");
     }
+    const uint32_t bits = static_cast<uint32_t>(q->c.bits) + 80u;
+    if (parts_applicable(q, p))
+    {
+        // s and p*e as one two-part transform, then b's draws and a in one
+        // kernel; the nonces are b's, s's and e's in the reference's order
+        const RngKey rng = ctx->rng();
+        const uint32_t kinds[2] = {part_ternary, part_scaled};
+        const uint32_t slots[2] = {1, 2};
+        uint32_t* const outs[2] = {s, e_poly};
+        if (int rc = run_parts(ctx, q, p, n, 1, 2, kinds, slots, outs, nullptr, nullptr))
+        {
+            return rc;
+        }
+        const cudaError_t e = q->kt->lhe_key(a, b, s, e_poly, n, rng, static_cast<int>((bits + 31) / 32),
+                                             bits % 32 ? (1u << (bits % 32)) - 1u : 0xffffffffu, !capturing(ctx),
+                                             q->h, ctx->stream);
+        if (e != cudaSuccess)
+        {
+            return cuda_fail(e, "launching the key combination");
+        }
+        ++ctx->launches;
+        nonce_add(ctx->nonce, 3 * n);
+        return HMPC_OK;
+    }
     int rc = hmpc_sample_uniform(ctx, q, n, 80, b);
-    // s and e are independent transforms; on the CUDA-core passes (no shared
-    // workspace) e's runs on the context's second stream meanwhile.  The
-    // nonces are taken on the host in the reference's order either way.
-    bool fork = false;
-    if (!rc)
-    {
-        std::lock_guard<std::mutex> lock(q->tables_mutex);
-        auto it = q->tile_choices.find(std::make_tuple(__builtin_ctzll(n), 0, static_cast<uint64_t>(1)));
-        const int radix = it == q->tile_choices.end() ? hmpc_modulus::TileChoice{}.radix_bits : it->second.radix_bits;
-        fork = radix != 0;
-    }
-    fork = fork && ctx->aux();
-    if (fork)
-    {
-        HMPC_CUDA(cudaEventRecord(ctx->fork_event, ctx->stream), "forking the key generation");
-        HMPC_CUDA(cudaStreamWaitEvent(ctx->aux_stream, ctx->fork_event, 0), "forking the key generation");
-    }
     if (!rc)
     {
         rc = run_transform(ctx, q, n, 1, false, producer_cbd, 1, 0, nullptr, s);
     }
     if (!rc)
     {
-        cudaStream_t main = ctx->stream;
-        if (fork)
-        {
-            ctx->stream = ctx->aux_stream;
-        }
         rc = run_transform(ctx, q, n, 1, false, producer_cbd, 20, 0, nullptr, e_poly);
-        ctx->stream = main;
-    }
-    if (fork)
-    {
-        HMPC_CUDA(cudaEventRecord(ctx->join_event, ctx->aux_stream), "joining the key generation");
-        HMPC_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->join_event, 0), "joining the key generation");
     }
     if (!rc)
     {

@@ -314,7 +314,7 @@ struct hmpc_ntt_batch
                 p.twiddles = inverse ? t->inverse : t->forward;
                 p.small_table = mod->small_table;
                 p.elements = degrees[i];
-                p.out = nullptr;
+                p.out[0] = nullptr;
                 p.src = nullptr;
                 index[i].push_back(static_cast<uint32_t>(params.size()));
                 params.push_back(p);
@@ -494,7 +494,7 @@ struct hmpc_ntt_batch
         for (size_t k = 0; k < params.size(); ++k)
         {
             const uint32_t i = param_poly[k];
-            h_params[k].out = out[i];
+            h_params[k].out[0] = out[i];
             h_params[k].src = param_pass[k] == 0 ? in[i] : nullptr;
         }
         HMPC_CUDA(cudaMemcpyAsync(d_params, h_params, params.size() * sizeof(PairPassParams), cudaMemcpyHostToDevice,

@@ -77,9 +77,15 @@ namespace hmpc_gb300
         cudaError_t (*ntt_batched)(const BatchedParams& bp, bool inverse, const HostModulus& m, unsigned grid,
                                    unsigned block, size_t smem, cudaStream_t stream);
         int (*ntt_batched_blocks_per_sm)(bool inverse, unsigned block, size_t smem);
+        // u, x, w: limb planes of `stride` words; dependent: launch with
+        // programmatic dependence on the kernel before it in the stream
         cudaError_t (*lhe_combine_pair)(uint32_t* c0, uint32_t* c1, const uint32_t* ka, const uint32_t* kb,
-                                        uint64_t n, const uint32_t* stacked, uint64_t elements,
-                                        const HostModulus& m, cudaStream_t stream);
+                                        uint64_t n, const uint32_t* u, const uint32_t* x, const uint32_t* w,
+                                        uint64_t stride, uint64_t elements, bool dependent, const HostModulus& m,
+                                        cudaStream_t stream);
+        cudaError_t (*lhe_key)(uint32_t* a, uint32_t* b, const uint32_t* s, const uint32_t* x, uint64_t elements,
+                               const RngKey& rng, int words, uint32_t top_mask, bool dependent, const HostModulus& m,
+                               cudaStream_t stream);
         // matrix-vector products (linalg.cuh)
         cudaError_t (*matvec)(uint32_t* z, const uint32_t* mat, const uint32_t* x, const MatvecParams& p,
                               const HostModulus& m, cudaStream_t stream);

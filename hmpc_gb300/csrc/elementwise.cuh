@@ -171,34 +171,60 @@ namespace hmpc_gb300
     // c0 = a * u + x and c1 = b * u + w with the key polynomials a, b broadcast
     // over the batch: the BGV combine when p * v (+ the lifted plaintext) and
     // p * w already went through the transform as inputs of their own
-    // (linearity of the NTT).  u, x, w are the three parts of one stacked
-    // transform output, [L][3 * elements]; u is read once for both products.
-    // One element per thread (about 50 registers at L = 8): enough resident
-    // warps to cover the loads' latency with the products' arithmetic.
-    // n is a power of two.
+    // (linearity of the NTT).  u, x and w have `stride` words per limb plane;
+    // u is read once for both products.  One element per thread (about 50
+    // registers at L = 8): enough resident warps to cover the loads' latency
+    // with the products' arithmetic.  n is a power of two.
     template<int L>
     __global__ void __launch_bounds__(256) lhe_combine_pair_kernel(uint32_t* c0, uint32_t* c1, const uint32_t* ka,
                                                                    const uint32_t* kb, uint64_t n,
-                                                                   const uint32_t* stacked, uint64_t elements,
-                                                                   const Modulus<L> m)
+                                                                   const uint32_t* u_planes,
+                                                                   const uint32_t* x_planes,
+                                                                   const uint32_t* w_planes, uint64_t stride,
+                                                                   uint64_t elements, const Modulus<L> m)
     {
-        const uint64_t stride = 3 * elements;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         const uint64_t mask = n - 1;
         for (uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < elements;
              e += static_cast<uint64_t>(gridDim.x) * blockDim.x)
         {
             uint32_t u[L], k[L], x[L];
-            load1<L>(u, stacked, stride, e);
+            load1<L>(u, u_planes, stride, e);
             load1<L>(k, ka, n, e & mask);
-            load1<L>(x, stacked + elements, stride, e);
+            load1<L>(x, x_planes, stride, e);
             mont_mul<L>(k, k, u, m);
             mod_add<L>(x, x, k, m);
             store1<L>(c0, elements, e, x);
             load1<L>(k, kb, n, e & mask);
-            load1<L>(x, stacked + 2 * elements, stride, e);
+            load1<L>(x, w_planes, stride, e);
             mont_mul<L>(k, k, u, m);
             mod_add<L>(x, x, k, m);
             store1<L>(c1, elements, e, x);
+        }
+    }
+
+    // The last node of a key pair: b uniform (element e from the generator at
+    // counter e, W words) and a = b * s + x, x the transform of p times the
+    // noise.
+    template<int L, int W>
+    __global__ void __launch_bounds__(256) lhe_key_kernel(uint32_t* a, uint32_t* b, const uint32_t* s,
+                                                          const uint32_t* x_planes, uint64_t elements,
+                                                          const RngKey rng, uint32_t top_mask, const Modulus<L> m)
+    {
+        const uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+        uint32_t w[W], k[L], x[L];
+        chacha_stream<W>(rng, static_cast<uint32_t>(e), w);
+        uniform_from_words<L, W, 0, W>(k, w, top_mask, m);
+        // b does not depend on the transforms: only the rest waits for them
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (e < elements)
+        {
+            store1<L>(b, elements, e, k);
+            load1<L>(x, s, elements, e);
+            mont_mul<L>(k, k, x, m);
+            load1<L>(x, x_planes, elements, e);
+            mod_add<L>(k, k, x, m);
+            store1<L>(a, elements, e, k);
         }
     }
 

@@ -116,23 +116,6 @@ struct hmpc_context
     // hook that makes one such wait run out (hmpc_context_set_test_wait)
     uint32_t tc_spin_limit = hmpc_gb300::detail::tc_default_spin_limit;
     uint32_t tc_test_stall = 0;
-    // a second stream for independent work of one call (fork / join events)
-    cudaStream_t aux_stream = nullptr;
-    cudaEvent_t fork_event = nullptr;
-    cudaEvent_t join_event = nullptr;
-
-    bool aux()
-    {
-        if (!aux_stream &&
-            (cudaStreamCreateWithFlags(&aux_stream, cudaStreamNonBlocking) != cudaSuccess ||
-             cudaEventCreateWithFlags(&fork_event, cudaEventDisableTiming) != cudaSuccess ||
-             cudaEventCreateWithFlags(&join_event, cudaEventDisableTiming) != cudaSuccess))
-        {
-            return false;
-        }
-        return true;
-    }
-
     // memory lent for the tensor-core digit buffers of the next calls instead
     // of the context's own (a serving lane's share of its server's pool, so
     // admission by memory counts it); nullptr: none
@@ -286,6 +269,13 @@ namespace hmpc_gb300::detail
     int run_plain(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, bool inverse, int kind,
                   uint32_t vx2, uint32_t security, const uint32_t* src, uint32_t* out);
     CastParams make_cast(const hmpc_modulus* dst, const hmpc_modulus* src);
+    bool capturing(const hmpc_context* ctx);
+    // BGV encryption on the CUDA cores from coefficient-form plaintexts, 3 *
+    // batch * n * L_q words of workspace; poly_rng: per-polynomial RNG
+    // descriptors of independent requests (the context's nonce stays)
+    int encrypt_cuda_cores(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n, uint64_t batch,
+                           const uint32_t* key_a, const uint32_t* key_b, const uint32_t* coefficients, uint32_t* c0,
+                           uint32_t* c1, uint32_t* workspace, const uint32_t* poly_rng, bool cuda_cores_only);
     // tensor-core engine: whether the modulus qualifies (2 to 8 limbs, q
     // below 0.996 * 2^(32L), top limb at least 32) and whether a call does
     // (forward from a tensor or CBD(V) samples, or inverse; at least 16

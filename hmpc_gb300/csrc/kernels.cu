@@ -51,9 +51,11 @@ namespace hmpc_gb300
             return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(g, 152ull * 64ull)));
         }
 
-        template<int Kind, int NW, bool Inverse>
-        cudaError_t launch_pair(const PairPassParams& p, const Modulus<L>& m, unsigned grid, unsigned block,
-                                size_t smem, cudaStream_t stream)
+        // dependent: with programmatic dependence on the kernel before it in the
+        // stream (the kernel waits for it by griddepcontrol.wait)
+        template<class... Params, class... Args>
+        cudaError_t launch(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, bool dependent,
+                           cudaStream_t stream, const Args&... args)
         {
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3(grid);
@@ -64,8 +66,15 @@ namespace hmpc_gb300
             attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
-            cfg.numAttrs = p.dependent ? 1u : 0u;
-            return cudaLaunchKernelEx(&cfg, ntt_pair_kernel<L, Kind, NW, Inverse>, p, m);
+            cfg.numAttrs = dependent ? 1u : 0u;
+            return cudaLaunchKernelEx(&cfg, kernel, args...);
+        }
+
+        template<int Kind, int NW, bool Inverse>
+        cudaError_t launch_pair(const PairPassParams& p, const Modulus<L>& m, unsigned grid, unsigned block,
+                                size_t smem, cudaStream_t stream)
+        {
+            return launch(ntt_pair_kernel<L, Kind, NW, Inverse>, grid, block, smem, p.dependent != 0, stream, p, m);
         }
 
         cudaError_t ntt_pair(const PairPassParams& p, int kind, int nw, bool inverse, const HostModulus& h,
@@ -90,6 +99,10 @@ namespace hmpc_gb300
                 case 4: return launch_pair<producer_cbd, 4, false>(p, m, grid, block, smem, stream);
                 default: return cudaErrorInvalidValue;
                 }
+            }
+            if (kind == producer_parts)
+            {
+                return launch_pair<producer_parts, 1, false>(p, m, grid, block, smem, stream);
             }
             if (kind == producer_uniform && nw == L + 2)
             {
@@ -345,16 +358,35 @@ namespace hmpc_gb300
         }
 
         cudaError_t lhe_combine_pair(uint32_t* c0, uint32_t* c1, const uint32_t* ka, const uint32_t* kb, uint64_t n,
-                                     const uint32_t* stacked, uint64_t elements, const HostModulus& h,
-                                     cudaStream_t stream)
+                                     const uint32_t* u, const uint32_t* x, const uint32_t* w, uint64_t stride,
+                                     uint64_t elements, bool dependent, const HostModulus& h, cudaStream_t stream)
         {
             if (elements == 0)
             {
                 return cudaSuccess;
             }
-            lhe_combine_pair_kernel<L><<<grid_for(elements, 256), 256, 0, stream>>>(c0, c1, ka, kb, n, stacked,
-                                                                                   elements, device_modulus(h));
-            return cudaGetLastError();
+            return launch(lhe_combine_pair_kernel<L>, grid_for(elements, 256), 256, 0, dependent, stream, c0, c1, ka,
+                          kb, n, u, x, w, stride, elements, device_modulus(h));
+        }
+
+        cudaError_t lhe_key(uint32_t* a, uint32_t* b, const uint32_t* s, const uint32_t* x, uint64_t elements,
+                            const RngKey& rng, int words, uint32_t top_mask, bool dependent, const HostModulus& h,
+                            cudaStream_t stream)
+        {
+            const unsigned block = elements >= 152ull * 256 ? 256 : 128;
+            const unsigned grid = static_cast<unsigned>((elements + block - 1) / block);
+            const Modulus<L> m = device_modulus(h);
+            if (words == L + 2)
+            {
+                return launch(lhe_key_kernel<L, L + 2>, grid, block, 0, dependent, stream, a, b, s, x, elements, rng,
+                              top_mask, m);
+            }
+            if (words == L + 3)
+            {
+                return launch(lhe_key_kernel<L, L + 3>, grid, block, 0, dependent, stream, a, b, s, x, elements, rng,
+                              top_mask, m);
+            }
+            return cudaErrorInvalidValue;
         }
 
         cudaError_t matvec(uint32_t* z, const uint32_t* mat, const uint32_t* x, const MatvecParams& p,
@@ -434,7 +466,7 @@ namespace hmpc_gb300
 
         const KernelTable table = {fma, binary, lhe_combine, uniform, cbd, to_montgomery,
                                    from_montgomery, cast, plain_stage, ct_mul, dec_combine, ntt_batched,
-                                   ntt_batched_blocks_per_sm, lhe_combine_pair, matvec, matvec_monomial,
+                                   ntt_batched_blocks_per_sm, lhe_combine_pair, lhe_key, matvec, matvec_monomial,
                                    reduce, equal, ntt_cluster, uniform_pairs, ntt_pair};
     }
 

@@ -112,53 +112,15 @@ extern "C" int hmpc_lhe_enc_noalloc(hmpc_context* ctx, hmpc_modulus* q, hmpc_mod
     }
     // every scratch word read below is written earlier in the same call, so
     // nothing has to be cleared
-    uint32_t* u = scratch;
-    uint32_t* v = scratch + poly_words;
-    uint32_t* msg = scratch + 2 * poly_words;
     uint32_t* coeff = scratch + 3 * poly_words;
-    // the reference's execution order: NTT(u), NTT(v), [INTT_p(x)],
-    // NTT_q(msg), c0, NTT(w), c1 (expr/cache.hpp:226-271)
-    int rc = run_transform(ctx, q, n, batch, false, producer_cbd, 1, 0, nullptr, u, nullptr, 0, true);
-    if (!rc)
-    {
-        rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v, nullptr, 0, true);
-    }
     const uint32_t* coefficients = plaintext;
-    if (!rc && plaintext_ntt)
+    if (plaintext_ntt)
     {
-        rc = run_transform(ctx, p, n, batch, true, producer_tensor, 0, 0, plaintext, coeff, nullptr, 0, true);
+        if (int rc = run_transform(ctx, p, n, batch, true, producer_tensor, 0, 0, plaintext, coeff, nullptr, 0, true))
+        {
+            return rc;
+        }
         coefficients = coeff;
     }
-    if (rc)
-    {
-        return rc;
-    }
-    cudaError_t e = q->kt->cast(msg, coefficients, elements, make_cast(q, p), q->h, ctx->stream);
-    if (e != cudaSuccess)
-    {
-        return cuda_fail(e, "launching cast");
-    }
-    ++ctx->launches;
-    if ((rc = run_transform(ctx, q, n, batch, false, producer_tensor, 0, 0, msg, msg, nullptr, 0, true)))
-    {
-        return rc;
-    }
-    const host::words pm = host::to_mont(q->c, p->c.q);
-    e = q->kt->lhe_combine(c0, key_a, n, u, v, msg, elements, pm.data(), q->h, ctx->stream);
-    if (e != cudaSuccess)
-    {
-        return cuda_fail(e, "launching combine");
-    }
-    ++ctx->launches;
-    if ((rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v, nullptr, 0, true)))  // w reuses v
-    {
-        return rc;
-    }
-    e = q->kt->lhe_combine(c1, key_b, n, u, v, nullptr, elements, pm.data(), q->h, ctx->stream);
-    if (e != cudaSuccess)
-    {
-        return cuda_fail(e, "launching combine");
-    }
-    ++ctx->launches;
-    return HMPC_OK;
+    return encrypt_cuda_cores(ctx, q, p, n, batch, key_a, key_b, coefficients, c0, c1, scratch, nullptr, true);
 }

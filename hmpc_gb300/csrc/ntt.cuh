@@ -17,22 +17,24 @@ namespace hmpc_gb300
         producer_tensor = 0,   // read `src` (or the output buffer when src == nullptr)
         producer_cbd = 1,      // centred binomial, 2V = vx2, NW words per sample
         producer_uniform = 2,  // uniform mod Q, W words per sample
+        producer_parts = 3,    // the parts of an encryption or key pair (PairParts)
     };
 
     // Generator key, nonce and counter of the stage-0 pair whose first element
     // is coefficient idx_u of polynomial `poly`.  With per-polynomial RNG
     // (batches of independent requests: p.poly_rng), polynomial i draws with
-    // nonce = desc[0..2] + rng_slot * desc[4] * N and counter = desc[3] * N +
+    // nonce = desc[0..2] + slot * desc[4] * N and counter = desc[3] * N +
     // coefficient, desc = poly_rng + 5 i -- exactly what the request would draw
     // alone with its own nonce.
     template<class Params>
-    __device__ __forceinline__ uint32_t pair_generator(const Params& p, uint64_t poly, uint64_t idx_u, RngKey& rng)
+    __device__ __forceinline__ uint32_t pair_generator(const Params& p, uint64_t poly, uint64_t idx_u, uint32_t slot,
+                                                       RngKey& rng)
     {
         rng = p.rng;
         if (p.poly_rng)
         {
             const uint32_t* d = p.poly_rng + poly * 5;
-            const uint64_t add = static_cast<uint64_t>(p.rng_slot) * d[4] << p.log_n;
+            const uint64_t add = static_cast<uint64_t>(slot) * d[4] << p.log_n;
             uint64_t s = static_cast<uint64_t>(d[0]) + static_cast<uint32_t>(add);
             rng.nonce[0] = static_cast<uint32_t>(s);
             s = static_cast<uint64_t>(d[1]) + static_cast<uint32_t>(add >> 32) + (s >> 32);
@@ -45,8 +47,7 @@ namespace hmpc_gb300
 
     template<int L, int Kind, int NW, class Params>
     __device__ __forceinline__ void produce_pair(const Params& p, const Modulus<L>& m, uint64_t poly,
-                                                 uint64_t idx_u, uint64_t idx_v, uint32_t (&u)[L],
-                                                 uint32_t (&v)[L])
+                                                 uint64_t idx_u, uint32_t (&u)[L], uint32_t (&v)[L])
     {
         if constexpr (Kind == producer_cbd)
         {
@@ -55,7 +56,7 @@ namespace hmpc_gb300
             // :316-329, comp/queue.hpp:191-212)
             uint32_t w[2 * NW];
             RngKey rng;
-            const uint32_t counter = pair_generator(p, poly, idx_u, rng);
+            const uint32_t counter = pair_generator(p, poly, idx_u, p.rng_slot, rng);
             chacha_stream<2 * NW>(rng, counter, w);
             int a = 0, b = 0;
             const int count = 2 * static_cast<int>(p.vx2);
@@ -77,14 +78,10 @@ namespace hmpc_gb300
         {
             uint32_t w[2 * NW];
             RngKey rng;
-            const uint32_t counter = pair_generator(p, poly, idx_u, rng);
+            const uint32_t counter = pair_generator(p, poly, idx_u, p.rng_slot, rng);
             chacha_stream<2 * NW>(rng, counter, w);
             uniform_from_words<L, NW, 0, 2 * NW>(u, w, p.top_mask, m);
             uniform_from_words<L, NW, NW, 2 * NW>(v, w, p.top_mask, m);
-        }
-        else
-        {
-            (void)idx_v;
         }
     }
 

@@ -36,14 +36,37 @@ namespace hmpc_gb300
 {
     constexpr uint32_t pair_max_threads = 512;
 
+    // Sampled transforms that run as one: part i is the polynomials
+    // [i * polys, (i + 1) * polys) of the pass and has an output buffer of its
+    // own.
+    constexpr int pair_max_parts = 3;
+
+    enum PairPartKind : uint32_t
+    {
+        part_ternary = 0,        // CBD(1/2)
+        part_scaled = 1,         // p * CBD(10)
+        part_scaled_message = 2, // p * CBD(10) + the centred lift of a residue mod p (one or two limbs)
+    };
+
+    struct PairParts
+    {
+        uint32_t kind[pair_max_parts];
+        uint32_t nonce[pair_max_parts][3];
+        const uint32_t* msg;           // msg_limbs planes of `elements` words, Montgomery form
+        uint32_t msg_limbs;
+        uint32_t pq[2], phalf[2], pninv;
+        uint32_t r2[9];                // R^2 mod Q
+    };
+
     struct PairPassParams
     {
-        uint32_t* out;                 // limb-planar, `elements` entries per limb
+        uint32_t* out[pair_max_parts]; // per part: limb-planar, `elements` entries per limb
+        uint64_t part_polys;           // polynomials of a part
         const uint32_t* src;           // tensor producer input (nullptr: read out)
         const uint32_t* twiddles;      // element-major [N][L]
         const uint32_t* small_table;   // Montgomery forms of 0..64, element-major
-        uint64_t elements;             // batch * N
-        uint64_t tiles;                // batch * tiles per polynomial
+        uint64_t elements;             // of one part: polynomials * N
+        uint64_t tiles;                // of all parts: polynomials * tiles per polynomial
         uint32_t log_n;
         uint32_t w, c;                 // stages of this pass, column bits
         uint32_t row_shift;            // element bit of the lowest row bit
@@ -52,8 +75,104 @@ namespace hmpc_gb300
         uint32_t top_mask;             // uniform producer: mask of the top word
         const uint32_t* poly_rng;      // per-polynomial RNG, see pair_generator
         uint32_t rng_slot;
-        uint32_t dependent;            // host side: programmatic dependence on the pass before
+        uint32_t dependent;            // host side: programmatic dependence on the kernel before
+        PairParts parts;               // parts producer
     };
+
+    // Canonical value of a residue mod p (one or two limbs, Montgomery form)
+    // lifted to the centred integer in (-p/2, p/2] (hmpc/ints/mod.hpp:259-307).
+    __device__ __forceinline__ int64_t centred_lift(const PairParts& p, uint32_t m0, uint32_t m1)
+    {
+        const uint64_t q = p.pq[0] | static_cast<uint64_t>(p.pq[1]) << 32;
+        const uint64_t half = p.phalf[0] | static_cast<uint64_t>(p.phalf[1]) << 32;
+        uint64_t v;
+        if (p.msg_limbs > 1)
+        {
+            unsigned __int128 t = (static_cast<uint64_t>(m1) << 32) | m0;
+            t += static_cast<unsigned __int128>(m0 * p.pninv) * q;  // the low word becomes 0
+            t >>= 32;
+            t += static_cast<unsigned __int128>(static_cast<uint32_t>(t) * p.pninv) * q;
+            t >>= 32;  // < 2q
+            v = static_cast<uint64_t>(t);
+            v = (t >> 64) != 0 || v >= q ? v - q : v;
+        }
+        else
+        {
+            v = (static_cast<uint64_t>(m0 * p.pninv) * p.pq[0] + m0) >> 32;  // <= q
+            v = v >= q ? v - q : v;
+        }
+        return v > half ? static_cast<int64_t>(v) - static_cast<int64_t>(q) : static_cast<int64_t>(v);
+    }
+
+    // r = x mod Q in Montgomery form, |x| < 2^70 < Q
+    template<int L>
+    __device__ __forceinline__ void int_to_mont(uint32_t (&r)[L], __int128 x, const uint32_t* r2, const Modulus<L>& m)
+    {
+        const bool negative = x < 0;
+        const unsigned __int128 a = static_cast<unsigned __int128>(negative ? -x : x);
+        uint32_t v[L], f[L];
+#pragma unroll
+        for (int j = 0; j < L; ++j)
+        {
+            v[j] = j < 3 ? static_cast<uint32_t>(a >> (32 * (j < 3 ? j : 0))) : 0u;
+            f[j] = r2[j];
+        }
+        mont_mul<L>(r, f, v, m);
+        if (negative)
+        {
+            mod_neg<L>(r, r, m);
+        }
+    }
+
+    // The stage-0 pair of a part: one generator, the lower element's draw first
+    // (number_theoretic_transform.hpp:316-329).  Both variances of BGV's
+    // samplers consume words 0 and 1 or 0 to 3 of one block.
+    template<int L>
+    __device__ __forceinline__ void produce_part_pair(const PairPassParams& p, const Modulus<L>& m, uint32_t part,
+                                                      uint64_t poly, uint32_t idx, uint32_t step, uint32_t (&u)[L],
+                                                      uint32_t (&v)[L])
+    {
+        const uint32_t kind = p.parts.kind[part];
+        uint32_t msg[2][2] = {};
+        if (kind == part_scaled_message)
+        {
+            // issued before the keystream is computed: their latency hides behind it
+            const uint32_t* at = p.parts.msg + (poly << p.log_n) + idx;
+            msg[0][0] = at[0];
+            msg[1][0] = at[step];
+            if (p.parts.msg_limbs > 1)
+            {
+                msg[0][1] = at[p.elements];
+                msg[1][1] = at[p.elements + step];
+            }
+        }
+        RngKey rng;
+        const uint32_t counter = pair_generator(p, poly, idx, part, rng);
+        if (!p.poly_rng)
+        {
+            rng.nonce[0] = p.parts.nonce[part][0];
+            rng.nonce[1] = p.parts.nonce[part][1];
+            rng.nonce[2] = p.parts.nonce[part][2];
+        }
+        uint32_t w[4];
+        chacha_stream<4>(rng, counter, w);
+        if (kind == part_ternary)
+        {
+            small_to_mont<L>(u, __popc(w[0] & 3u) - 1, p.small_table, m);
+            small_to_mont<L>(v, __popc(w[1] & 3u) - 1, p.small_table, m);
+            return;
+        }
+        const uint64_t scale = p.parts.pq[0] | static_cast<uint64_t>(p.parts.pq[1]) << 32;
+        __int128 x = static_cast<__int128>(scale) * (__popc(w[0]) + __popc(w[1] & 0xffu) - 20);
+        __int128 y = static_cast<__int128>(scale) * (__popc(w[2]) + __popc(w[3] & 0xffu) - 20);
+        if (kind == part_scaled_message)
+        {
+            x += centred_lift(p.parts, msg[0][0], msg[0][1]);
+            y += centred_lift(p.parts, msg[1][0], msg[1][1]);
+        }
+        int_to_mont<L>(u, x, p.parts.r2, m);
+        int_to_mont<L>(v, y, p.parts.r2, m);
+    }
 
     // One pass over the tiles of block `block` of the pass's grid.  exchange
     // holds [2][L][blockDim.x] words.  Wait: whether the input may still be
@@ -70,7 +189,18 @@ namespace hmpc_gb300
         const uint32_t col = t & ((1u << c) - 1u);
         const uint32_t r = (t >> c) & ((1u << (w - 1)) - 1u);  // the row bits but the pair's
         const uint32_t tile_bits = p.log_n - w - c;
-        const uint64_t poly = tile >> tile_bits;
+        uint64_t poly = tile >> tile_bits;
+        uint32_t part = 0;
+#pragma unroll
+        for (int i = 1; i < pair_max_parts; ++i)
+        {
+            if (poly >= p.part_polys)
+            {
+                poly -= p.part_polys;
+                ++part;
+            }
+        }
+        uint32_t* const out_part = p.out[part];
         const uint32_t in_poly = static_cast<uint32_t>(tile) & ((1u << tile_bits) - 1u);
         const uint32_t mid_bits = p.row_shift - c;
         const uint32_t high = in_poly >> mid_bits;  // index bits above the rows
@@ -97,7 +227,14 @@ namespace hmpc_gb300
             {
                 if (active)
                 {
-                    produce_pair<L, Kind, NW>(p, m, poly, idx, idx + step, lo, hi);
+                    if constexpr (Kind == producer_parts)
+                    {
+                        produce_part_pair<L>(p, m, part, poly, idx, step, lo, hi);
+                    }
+                    else
+                    {
+                        produce_pair<L, Kind, NW>(p, m, poly, idx, lo, hi);
+                    }
                 }
                 else
                 {
@@ -107,7 +244,7 @@ namespace hmpc_gb300
             }
             else
             {
-                const uint32_t* in = (p.src ? p.src : p.out) + poly_base + idx;
+                const uint32_t* in = (p.src ? p.src : out_part) + poly_base + idx;
 #pragma unroll
                 for (int j = 0; j < L; ++j)
                 {
@@ -200,7 +337,7 @@ namespace hmpc_gb300
         {
             const uint32_t row = Inverse ? r : r << 1;
             const uint32_t step = 1u << (p.row_shift + (Inverse ? w - 1 : 0u));
-            uint32_t* out = p.out + poly_base + (base | (row << p.row_shift));
+            uint32_t* out = out_part + poly_base + (base | (row << p.row_shift));
 #pragma unroll
             for (int j = 0; j < L; ++j)
             {

@@ -55,7 +55,7 @@ namespace hmpc_gb300
                 q.vx2 = p.vx2;
                 q.top_mask = p.top_mask;
                 q.small_table = p.small_table;
-                produce_pair<L, Kind, NW>(q, m, poly, target, target + step, u, v);
+                produce_pair<L, Kind, NW>(q, m, poly, target, u, v);
             }
             else
             {

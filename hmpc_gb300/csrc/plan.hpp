@@ -70,6 +70,7 @@ namespace hmpc_gb300
             PairPlan pp{};
             PairPassParams& p = pp.params;
             p.log_n = static_cast<uint32_t>(log_n);
+            p.part_polys = batch;
             p.w = static_cast<uint32_t>(rg.hi - rg.lo);
             p.c = static_cast<uint32_t>(rg.c);
             p.row_shift = static_cast<uint32_t>(rg.lo);

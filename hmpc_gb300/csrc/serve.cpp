@@ -312,10 +312,7 @@ struct hmpc_server
         const int lp = k.p->c.limbs;
         const uint64_t total = n * polys;
         const uint64_t qw = total * static_cast<uint64_t>(lq);
-        uint32_t* u = scratch;
-        uint32_t* v = u + qw;
-        uint32_t* msg = v + qw;
-        uint32_t* pt = msg + qw;
+        uint32_t* pt = scratch + 3 * qw;
         uint32_t* c0 = pt + total * static_cast<uint64_t>(lp);
         uint32_t* c1 = c0 + qw;
         uint32_t* host_desc = lane_desc[static_cast<size_t>(d.lane)];
@@ -349,40 +346,11 @@ struct hmpc_server
         }
         uint32_t* out0 = single ? r0.out0 : c0;
         uint32_t* out1 = single ? r0.out1 : c1;
-        int rc = run_transform(lane, k.q, n, polys, false, producer_cbd, 1, 0, nullptr, u, dev_desc, 0);
-        if (!rc)
-        {
-            rc = run_transform(lane, k.q, n, polys, false, producer_cbd, 20, 0, nullptr, v, dev_desc, 1);
-        }
-        if (rc)
+        if (int rc = encrypt_cuda_cores(lane, k.q, k.p, n, polys, k.a, k.b, plaintext, out0, out1, scratch, dev_desc,
+                                        false))
         {
             return rc;
         }
-        cudaError_t e = k.q->kt->cast(msg, plaintext, total, make_cast(k.q, k.p), k.q->h, s);
-        if (e != cudaSuccess)
-        {
-            return cuda_fail(e, "launching cast");
-        }
-        ++lane->launches;
-        if ((rc = run_transform(lane, k.q, n, polys, false, producer_tensor, 0, 0, msg, msg)))
-        {
-            return rc;
-        }
-        const host::words pm = host::to_mont(k.q->c, k.p->c.q);
-        if ((e = k.q->kt->lhe_combine(out0, k.a, n, u, v, msg, total, pm.data(), k.q->h, s)) != cudaSuccess)
-        {
-            return cuda_fail(e, "launching combine");
-        }
-        ++lane->launches;
-        if ((rc = run_transform(lane, k.q, n, polys, false, producer_cbd, 20, 0, nullptr, v, dev_desc, 2)))
-        {
-            return rc;
-        }
-        if ((e = k.q->kt->lhe_combine(out1, k.b, n, u, v, nullptr, total, pm.data(), k.q->h, s)) != cudaSuccess)
-        {
-            return cuda_fail(e, "launching combine");
-        }
-        ++lane->launches;
         if (!single)
         {
             uint64_t at = 0;
