@@ -255,7 +255,6 @@ namespace hmpc_gb300::detail
             cp.src_half[j] = src->c.half[static_cast<size_t>(j)];
         }
         const int nw = std::max(ls, ld) + 1;
-        cp.norm_words = static_cast<uint32_t>(nw);
         host::words offset;
         if (host::compare(dst->c.q, src->c.q) > 0)
         {

@@ -205,6 +205,6 @@ namespace hmpc_gb300
             v[i] = w[First + i];
         }
         v[W - 1] &= top_mask;
-        redc_wide<L, W>(r, v, m);
+        redc<L, W>(r, v, m);
     }
 }

@@ -40,7 +40,6 @@ namespace hmpc_gb300
         uint32_t src_q[max_device_limbs];
         uint32_t src_half[max_device_limbs];
         uint32_t offset[max_device_limbs + 1];  // added when the value exceeds src/2
-        uint32_t norm_words;                      // words of value + offset
         uint32_t direct;                          // 1: value + offset < target Q
         uint32_t factor[max_device_limbs];        // R^2 (direct) or R'*R^2 mod Q
     };

@@ -370,7 +370,7 @@ namespace hmpc_gb300
         }
     }
 
-    // Montgomery form -> canonical integer: mont_mul(x, 1) (mod.hpp:356-361)
+    // Montgomery form -> canonical integer (mod.hpp:356-361)
     template<int L>
     __global__ void __launch_bounds__(256) from_montgomery_kernel(uint32_t* out, const uint32_t* in,
                                                                   uint64_t elements, const Modulus<L> m)
@@ -380,10 +380,8 @@ namespace hmpc_gb300
         {
             uint32_t x[L], o[L];
             load1<L>(x, in, elements, e);
-            set_zero<L>(o);
-            o[0] = 1u;
-            mont_mul<L>(x, x, o, m);
-            store1<L>(out, elements, e, x);
+            redc<L, L>(o, x, m);
+            store1<L>(out, elements, e, o);
         }
     }
 }

@@ -263,7 +263,21 @@ namespace hmpc_gb300
             {
                 return cudaSuccess;
             }
-            cast_kernel<L><<<grid_for(elements, 256), 256, 0, stream>>>(out, in, elements, cp, device_modulus(h));
+            const unsigned grid = grid_for(elements, 256);
+            const Modulus<L> m = device_modulus(h);
+            switch (cp.src_limbs)
+            {
+            case 1: cast_kernel<L, 1><<<grid, 256, 0, stream>>>(out, in, elements, cp, m); break;
+            case 2: cast_kernel<L, 2><<<grid, 256, 0, stream>>>(out, in, elements, cp, m); break;
+            case 3: cast_kernel<L, 3><<<grid, 256, 0, stream>>>(out, in, elements, cp, m); break;
+            case 4: cast_kernel<L, 4><<<grid, 256, 0, stream>>>(out, in, elements, cp, m); break;
+            case 5: cast_kernel<L, 5><<<grid, 256, 0, stream>>>(out, in, elements, cp, m); break;
+            case 6: cast_kernel<L, 6><<<grid, 256, 0, stream>>>(out, in, elements, cp, m); break;
+            case 7: cast_kernel<L, 7><<<grid, 256, 0, stream>>>(out, in, elements, cp, m); break;
+            case 8: cast_kernel<L, 8><<<grid, 256, 0, stream>>>(out, in, elements, cp, m); break;
+            case 9: cast_kernel<L, 9><<<grid, 256, 0, stream>>>(out, in, elements, cp, m); break;
+            default: return cudaErrorInvalidValue;
+            }
             return cudaGetLastError();
         }
 

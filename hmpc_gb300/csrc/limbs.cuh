@@ -5,7 +5,7 @@
 // representation as hmpc's mod<Q> (hmpc/ints/mod.hpp:73-193), so any exact
 // implementation of the operations below reproduces the reference bit for bit.
 //
-// Additions, subtractions and the wide reduction use PTX carry chains
+// Additions, subtractions and products use PTX carry chains
 // (add.cc / addc / sub.cc / subc / mad.lo.cc / madc.hi.cc); each chain is a run
 // of consecutive volatile asm statements with no other instruction between
 // them touching the condition code.  The Montgomery product keeps its running
@@ -342,63 +342,45 @@ namespace hmpc_gb300
         reduce_once<L>(r, t, m);
     }
 
-    // Reduction of a W-word value with R' = 2^(32W) (hmpc/core/num/modulo.hpp
-    // :30-66 with auxiliary power W); used by the uniform sampler
-    // (hmpc/ints/mod.hpp:210-215), where W >= L.
+    // r = v * 2^(-32W) mod Q, fully reduced, for any W-word value: the reduction
+    // with auxiliary power W (hmpc/core/num/modulo.hpp:30-66) -- W = L turns a
+    // Montgomery form into the canonical value (hmpc/ints/mod.hpp:356-361), the
+    // uniform sampler reduces W > L words (mod.hpp:210-215).  The rows of
+    // mont_mul's reduction on a window of L + 2 words that takes in the value's
+    // next word after each shift.
     template<int L, int W>
-    __device__ __forceinline__ void redc_wide(uint32_t (&r)[L], const uint32_t (&v)[W], const Modulus<L>& m)
+    __device__ __forceinline__ void redc(uint32_t (&r)[L], const uint32_t (&v)[W], const Modulus<L>& m)
     {
-        uint32_t t[W + L + 1];
+        Columns<L> c;
+        auto word = [&](int j) { return j < W ? v[j < W ? j : 0] : 0u; };
 #pragma unroll
-        for (int j = 0; j < W; ++j)
+        for (int j = 0; j < Columns<L>::EW; ++j)
         {
-            t[j] = v[j];
+            c.even[j] = word(j);
         }
 #pragma unroll
-        for (int j = W; j < W + L + 1; ++j)
+        for (int j = 0; j < Columns<L>::OW; ++j)
         {
-            t[j] = 0u;
+            c.odd[j] = j + 1 >= Columns<L>::EW ? word(j + 1) : 0u;
         }
+        c.top = 0u;
+        c.pending = 0u;
 #pragma unroll
         for (int i = 0; i < W; ++i)
         {
-            const uint32_t mq = t[i] * m.ninv;
-            t[i] = ptx::mad_lo_cc(mq, m.q[0], t[i]);
-#pragma unroll
-            for (int j = 1; j < L; ++j)
+            const uint32_t mq = (c.even[0] + c.pending) * m.ninv;
+            c.template add_product<true>(m.q, mq);
+            c.shift();
+            if (i + 1 + L < W)
             {
-                t[i + j] = ptx::madc_lo_cc(mq, m.q[j], t[i + j]);
-            }
-#pragma unroll
-            for (int k = i + L; k < W + L + 1; ++k)
-            {
-                t[k] = ptx::addc_cc(t[k], 0u);
-            }
-            t[i + 1] = ptx::mad_hi_cc(mq, m.q[0], t[i + 1]);
-#pragma unroll
-            for (int j = 1; j < L; ++j)
-            {
-                t[i + j + 1] = ptx::madc_hi_cc(mq, m.q[j], t[i + j + 1]);
-            }
-#pragma unroll
-            for (int k = i + L + 1; k < W + L + 1; ++k)
-            {
-                t[k] = ptx::addc_cc(t[k], 0u);
+                uint32_t& last = L % 2 == 0 ? c.odd[L > 1 ? L - 1 : 0] : c.even[L % 2 ? L : 0];
+                last = ptx::add_cc(last, word(i + 1 + L));
+                c.top = ptx::addc(0u, 0u);
             }
         }
-        uint32_t d[L];
-        d[0] = ptx::sub_cc(t[W], m.q[0]);
-#pragma unroll
-        for (int j = 1; j < L; ++j)
-        {
-            d[j] = ptx::subc_cc(t[W + j], m.q[j]);
-        }
-        uint32_t borrow = ptx::subc(t[W + L], 0u);
-#pragma unroll
-        for (int j = 0; j < L; ++j)
-        {
-            r[j] = borrow ? t[W + j] : d[j];
-        }
+        uint32_t t[L + 1];
+        c.value(t);
+        reduce_once<L>(r, t, m);
     }
 
     template<int L>
