@@ -93,6 +93,10 @@ namespace hmpc_gb300
         // one level of a reduction into `grid` values (mod: mod<Q> with m, else uint with top_mask)
         cudaError_t (*reduce)(uint32_t* out, const uint32_t* in, uint64_t elements, int op, bool mod,
                               uint32_t top_mask, unsigned grid, const HostModulus& m, cudaStream_t stream);
+        // sum mod Q of fewer than 2^32 residues: limbs * chunks 64-bit partial
+        // sums in `part`, then one block; dependent: as for lhe_combine_pair
+        cudaError_t (*plane_sum)(uint32_t* out, uint64_t* part, const uint32_t* in, uint64_t elements,
+                                 unsigned chunks, bool dependent, const HostModulus& m, cudaStream_t stream);
         cudaError_t (*equal)(uint32_t* out, const uint32_t* a, const uint32_t* b, uint64_t elements,
                              cudaStream_t stream);
         // one thread-block cluster per polynomial (cluster.cuh), degrees 2^10..2^14

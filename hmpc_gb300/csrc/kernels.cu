@@ -443,6 +443,19 @@ namespace hmpc_gb300
             return cudaGetLastError();
         }
 
+        cudaError_t plane_sum(uint32_t* out, uint64_t* part, const uint32_t* in, uint64_t elements, unsigned chunks,
+                              bool dependent, const HostModulus& h, cudaStream_t stream)
+        {
+            plane_sum_kernel<L><<<L * chunks, 256, 0, stream>>>(part, in, elements, chunks);
+            cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess)
+            {
+                return e;
+            }
+            return launch(plane_sum_finish_kernel<L>, 1, 32 * L, 0, dependent, stream, out, part, chunks,
+                          holder(h.r2), device_modulus(h));
+        }
+
         cudaError_t equal(uint32_t* out, const uint32_t* a, const uint32_t* b, uint64_t elements,
                           cudaStream_t stream)
         {
@@ -481,7 +494,7 @@ namespace hmpc_gb300
         const KernelTable table = {fma, binary, lhe_combine, uniform, cbd, to_montgomery,
                                    from_montgomery, cast, plain_stage, ct_mul, dec_combine, ntt_batched,
                                    ntt_batched_blocks_per_sm, lhe_combine_pair, lhe_key, matvec, matvec_monomial,
-                                   reduce, equal, ntt_cluster, uniform_pairs, ntt_pair};
+                                   reduce, plane_sum, equal, ntt_cluster, uniform_pairs, ntt_pair};
     }
 
     const KernelTable* HMPC_CAT(kernel_table_, HMPC_L)()

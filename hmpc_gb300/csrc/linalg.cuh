@@ -365,6 +365,139 @@ namespace hmpc_gb300
         }
     }
 
+    // Sums of mod<Q> values, first level.  The sum of multi-limb integers is the
+    // sum over the limb planes of 2^(32 j) times the plane's own sum, so each
+    // plane is summed by itself in 64 bits (fewer than 2^32 elements), two
+    // additions for each word, and reduced mod Q once at the end.  Planes start at
+    // any word (an odd number of elements): a plane's 16-byte aligned middle is
+    // read by 128-bit loads, eight in flight per thread.  Bound by HBM: 9,999,991
+    // residues of 4 limbs (160 MB) 56.8 us folding each residue mod Q from scalar
+    // loads, 28.3 us so, both launches.  Block (plane, chunk) writes one partial sum.
+    template<int L>
+    __global__ void __launch_bounds__(256) plane_sum_kernel(uint64_t* part, const uint32_t* in, uint64_t elements,
+                                                            uint32_t chunks)
+    {
+        __shared__ uint64_t sums[8];
+        const uint32_t plane = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
+        const uint32_t* p = in + plane * elements;
+        const uint64_t skew = (4u - (static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p)) >> 2)) & 3u;
+        const uint64_t head = skew < elements ? skew : elements;
+        const uint64_t quads = (elements - head) / 4;
+        const uint4* q = reinterpret_cast<const uint4*>(p + head);
+        const uint64_t threads = static_cast<uint64_t>(chunks) * blockDim.x;
+        const uint64_t tid = static_cast<uint64_t>(chunk) * blockDim.x + threadIdx.x;
+        uint64_t acc = 0;
+        constexpr int depth = 8;
+        uint64_t i = tid;
+        for (; i + (depth - 1) * threads < quads; i += depth * threads)
+        {
+            uint4 v[depth];
+#pragma unroll
+            for (int k = 0; k < depth; ++k)
+            {
+                v[k] = __ldcs(q + i + k * threads);
+            }
+#pragma unroll
+            for (int k = 0; k < depth; ++k)
+            {
+                acc += static_cast<uint64_t>(v[k].x) + v[k].y;
+                acc += static_cast<uint64_t>(v[k].z) + v[k].w;
+            }
+        }
+        for (; i < quads; i += threads)
+        {
+            const uint4 v = __ldcs(q + i);
+            acc += static_cast<uint64_t>(v.x) + v.y;
+            acc += static_cast<uint64_t>(v.z) + v.w;
+        }
+        // the words before the first and after the last aligned quad
+        if (tid < head)
+        {
+            acc += p[tid];
+        }
+        if (tid < elements - head - 4 * quads)
+        {
+            acc += p[head + 4 * quads + tid];
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+        {
+            acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        }
+        if ((threadIdx.x & 31u) == 0)
+        {
+            sums[threadIdx.x >> 5] = acc;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            for (uint32_t w = 1; w < blockDim.x >> 5; ++w)
+            {
+                acc += sums[w];
+            }
+            part[blockIdx.x] = acc;
+        }
+    }
+
+    // Second level, one warp per plane: the plane's sum from its chunks, then
+    // the L + 2 word integer sum_j 2^(32 j) S_j mod Q by Horner's rule in base
+    // R (r2 holds R^2 mod Q, m.one R mod Q).
+    template<int L>
+    __global__ void __launch_bounds__(32 * L) plane_sum_finish_kernel(uint32_t* out, const uint64_t* part,
+                                                                      uint32_t chunks, const Modulus<L> r2,
+                                                                      const Modulus<L> m)
+    {
+        __shared__ uint64_t sums[L];
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const uint32_t plane = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+        uint64_t acc = 0;
+        for (uint32_t k = lane; k < chunks; k += 32)
+        {
+            acc += part[plane * chunks + k];
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+        {
+            acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        }
+        if (lane == 0)
+        {
+            sums[plane] = acc;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            constexpr int groups = (L + 2 + L - 1) / L;  // base-R digits
+            uint32_t v[groups * L];
+            uint64_t carry = 0;  // below 2^33: the next plane's sum shifted in
+            uint64_t high = 0;
+#pragma unroll
+            for (int j = 0; j < groups * L; ++j)
+            {
+                const uint64_t s = j < L ? sums[j < L ? j : 0] : 0u;
+                carry += (s & 0xffffffffu) + high;
+                high = s >> 32;
+                v[j] = static_cast<uint32_t>(carry);
+                carry >>= 32;
+            }
+            uint32_t r[L], d[L];
+            set_zero<L>(r);
+#pragma unroll
+            for (int g = groups - 1; g >= 0; --g)
+            {
+#pragma unroll
+                for (int j = 0; j < L; ++j)
+                {
+                    d[j] = v[g * L + j];
+                }
+                mont_mul<L>(d, m.one, d, m);  // d mod Q
+                mont_mul<L>(r, r2.one, r, m); // r * R
+                mod_add<L>(r, r, d, m);
+            }
+            store1<L>(out, 1, 0, r);
+        }
+    }
+
     // out[e] = 1 if every limb of a[e] and b[e] agrees, else 0: the hmpc::bit
     // of x == y (expr/binary_expression.hpp with core/equal_to.hpp)
     template<int L>
