@@ -347,8 +347,9 @@ namespace hmpc_gb300
     // Montgomery form into the canonical value (hmpc/ints/mod.hpp:356-361), the
     // uniform sampler reduces W > L words (mod.hpp:210-215).  The rows of
     // mont_mul's reduction on a window of L + 2 words that takes in the value's
-    // next word after each shift.
-    template<int L, int W>
+    // next word after each shift.  With fewer Rows, r = v * 2^(-32 Rows) mod Q
+    // for v < Q * 2^(32 Rows).
+    template<int L, int W, int Rows = W>
     __device__ __forceinline__ void redc(uint32_t (&r)[L], const uint32_t (&v)[W], const Modulus<L>& m)
     {
         Columns<L> c;
@@ -366,7 +367,7 @@ namespace hmpc_gb300
         c.top = 0u;
         c.pending = 0u;
 #pragma unroll
-        for (int i = 0; i < W; ++i)
+        for (int i = 0; i < Rows; ++i)
         {
             const uint32_t mq = (c.even[0] + c.pending) * m.ninv;
             c.template add_product<true>(m.q, mq);
@@ -381,6 +382,72 @@ namespace hmpc_gb300
         uint32_t t[L + 1];
         c.value(t);
         reduce_once<L>(r, t, m);
+    }
+
+    // t = (t + a * b) mod Q * R for t < Q * R and a, b < Q: one term of a sum of
+    // products that is reduced once (redc<L, 2L, L>), so a term costs the L^2
+    // wide multiply-adds of its product instead of a Montgomery product's
+    // 2 L^2 + L.  The product is formed on two sums of 64-bit columns, as in
+    // Columns, with every carry out of a row in the next column's low word.
+    template<int L>
+    __device__ __forceinline__ void add_product(uint32_t (&t)[2 * L], const uint32_t (&a)[L], const uint32_t (&b)[L],
+                                                const Modulus<L>& m)
+    {
+        // [0]: columns at words 0, 2, ...; [1]: at words 1, 3, ...
+        uint32_t columns[2][2 * L + 1];
+#pragma unroll
+        for (int k = 0; k < 2 * L + 1; ++k)
+        {
+            columns[0][k] = 0u;
+            columns[1][k] = 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < L; ++i)
+        {
+#pragma unroll
+            for (int parity = 0; parity < 2; ++parity)
+            {
+                uint32_t (&c)[2 * L + 1] = columns[parity];
+                const int first = (i + parity) % 2;
+#pragma unroll
+                for (int j = first; j < L; j += 2)
+                {
+                    c[i + j] = j == first ? ptx::mad_lo_cc(a[j], b[i], c[i + j]) : ptx::madc_lo_cc(a[j], b[i], c[i + j]);
+                    c[i + j + 1] = ptx::madc_hi_cc(a[j], b[i], c[i + j + 1]);
+                    if (j + 2 >= L && i + j + 2 < 2 * L)
+                    {
+                        c[i + j + 2] = ptx::addc(c[i + j + 2], 0u);
+                    }
+                }
+            }
+        }
+        t[0] = ptx::add_cc(t[0], columns[0][0]);
+#pragma unroll
+        for (int k = 1; k < 2 * L; ++k)
+        {
+            t[k] = ptx::addc_cc(t[k], columns[0][k]);
+        }
+        uint32_t high[L + 1];
+        high[L] = ptx::addc(0u, 0u);
+        t[1] = ptx::add_cc(t[1], columns[1][1]);
+#pragma unroll
+        for (int k = 2; k < 2 * L; ++k)
+        {
+            t[k] = ptx::addc_cc(t[k], columns[1][k]);
+        }
+        high[L] = ptx::addc(high[L], 0u);
+        uint32_t r[L];
+#pragma unroll
+        for (int k = 0; k < L; ++k)
+        {
+            high[k] = t[L + k];
+        }
+        reduce_once<L>(r, high, m);
+#pragma unroll
+        for (int k = 0; k < L; ++k)
+        {
+            t[L + k] = r[k];
+        }
     }
 
     template<int L>
