@@ -229,9 +229,12 @@ namespace hmpc_gb300
     }
 
     // ciphertext x ciphertext in NTT form: the tensor product
-    // (d0, d1, d2) = (a0*b0, a0*b1 + a1*b0, a1*b1).  No counterpart in the
-    // reference, whose ciphertexts only support linear operations
-    // (expr/crypto/lhe/ciphertext.hpp:49-81).
+    // (d0, d1, d2) = (a0*b0, a0*b1 + a1*b0, a1*b1), the middle one as
+    // (a0 + a1)(b0 + b1) - d0 - d2: three products instead of four.  No
+    // counterpart in the reference, whose ciphertexts only support linear
+    // operations (expr/crypto/lhe/ciphertext.hpp:49-81).  Bound by the products
+    // above 4 limbs: 2^21 elements of 8 limbs 188 -> 117 us (3.9 TB/s), 12 * 2^14
+    // of 7 limbs 18.5 -> 12.5 us, with the faster Montgomery product.
     template<int L>
     __global__ void __launch_bounds__(256) ct_mul_kernel(uint32_t* d0, uint32_t* d1, uint32_t* d2,
                                                          const uint32_t* a0, const uint32_t* a1, const uint32_t* b0,
@@ -240,19 +243,21 @@ namespace hmpc_gb300
         for (uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < elements;
              e += static_cast<uint64_t>(gridDim.x) * blockDim.x)
         {
-            uint32_t x0[L], x1[L], y0[L], y1[L], r[L], t[L];
+            uint32_t x0[L], x1[L], y0[L], y1[L], s[L], t[L];
             load1<L>(x0, a0, elements, e);
             load1<L>(x1, a1, elements, e);
             load1<L>(y0, b0, elements, e);
             load1<L>(y1, b1, elements, e);
-            mont_mul<L>(r, x0, y0, m);
-            store1<L>(d0, elements, e, r);
-            mont_mul<L>(r, x0, y1, m);
-            mont_mul<L>(t, x1, y0, m);
-            mod_add<L>(r, r, t, m);
-            store1<L>(d1, elements, e, r);
-            mont_mul<L>(r, x1, y1, m);
-            store1<L>(d2, elements, e, r);
+            mod_add<L>(s, x0, x1, m);
+            mod_add<L>(t, y0, y1, m);
+            mont_mul<L>(x0, x0, y0, m);
+            store1<L>(d0, elements, e, x0);
+            mont_mul<L>(x1, x1, y1, m);
+            store1<L>(d2, elements, e, x1);
+            mont_mul<L>(s, s, t, m);
+            mod_sub<L>(s, s, x0, m);
+            mod_sub<L>(s, s, x1, m);
+            store1<L>(d1, elements, e, s);
         }
     }
 
