@@ -7,6 +7,7 @@ operation runs through the C ABI of libhmpc_gb300.so; PyTorch only provides
 device memory and the stream.
 """
 import ctypes
+import math
 import os
 
 import numpy as np
@@ -104,15 +105,17 @@ class Tensor:
         self.modulus = modulus
         self.shape = tuple(int(s) for s in shape)
         self.n = int(n)
-        self.elements = int(np.prod(self.shape, dtype=np.int64)) * self.n
+        self.elements = math.prod(self.shape) * self.n
         if data is None:
             data = torch.empty((modulus.limbs, self.elements), dtype=torch.int32, device=modulus.queue.device)
-        assert data.dtype == torch.int32 and data.shape == (modulus.limbs, self.elements) and data.is_contiguous()
+        else:
+            assert data.dtype == torch.int32 and data.is_contiguous()
+            assert data.shape == (modulus.limbs, self.elements)
         self.data = data
 
     @property
     def batch(self):
-        return int(np.prod(self.shape, dtype=np.int64))
+        return math.prod(self.shape)
 
     def numpy(self):
         return self.data.cpu().numpy().view(np.uint32)
