@@ -1288,12 +1288,16 @@ int hmpc_lhe_enc(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n
     const uint64_t lq = static_cast<uint64_t>(q->c.limbs);
     const uint64_t lp = static_cast<uint64_t>(p->c.limbs);
     const uint64_t poly_words = elements * lq;
-    uint32_t* ws = ctx->scratch(3 * poly_words + (plaintext_ntt ? elements * lp : 0));
+    const int tc_splits = tc_plan_splits(q, n, batch);
+    const bool tensor = tc_splits && n >= 16 && tc_supported(q) && p->c.limbs <= 2;
+    // the tensor-core plan's last stages write the ciphertext themselves
+    const uint64_t ws_words = tensor && tc_tail(q, n, false) ? 0 : 3 * poly_words;
+    uint32_t* ws = ctx->scratch(std::max<uint64_t>(1, ws_words + (plaintext_ntt ? elements * lp : 0)));
     if (!ws)
     {
         return fail(HMPC_ERROR_OUT_OF_MEMORY, "allocating the encryption workspace");
     }
-    uint32_t* coeff = ws + 3 * poly_words;
+    uint32_t* coeff = ws + ws_words;
     const uint32_t* coefficients = plaintext;
     if (plaintext_ntt)
     {
@@ -1303,16 +1307,15 @@ int hmpc_lhe_enc(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n
         }
         coefficients = coeff;
     }
-    const int tc_splits = tc_plan_splits(q, n, batch);
-    if (tc_splits && n >= 16 && tc_supported(q) && p->c.limbs <= 2)
+    if (tensor)
     {
         // Tensor-core plan for q: the NTT is linear, so p*NTT(v) + NTT(lift(m))
         // is one transform of the small integers p*v + lift(m) drawn and lifted
         // in its first group, and p*NTT(w) one of p*w.  The three transforms
         // (u, p*v + lift(m), p*w) share every constant after their first
         // group, so they run stacked: three first-group launches, then the
-        // other groups once over 3 * batch polynomials.  One combine reads u
-        // once and writes c0 and c1; every result is the reduced
+        // other groups once over 3 * batch polynomials, the last stages'
+        // kernel writing c0 and c1.  Every result is the reduced
         // representative, so the ciphertext is the reference's bit for bit.  RNG order as the
         // reference's plan: u, v, w (expr/cache.hpp:226-271).
         const TcSmallInput with_msg{coefficients, p};
@@ -1323,20 +1326,7 @@ int hmpc_lhe_enc(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n
         parts[1].small = &with_msg;
         parts[2].vx2 = 20;
         parts[2].small = &no_msg;
-        uint32_t* stacked = ws;  // [L][3 * elements]: u | p*v + lift(m) | p*w, in NTT form
-        int rc = run_tc_stacked(ctx, q, n, batch, parts, 3, stacked, tc_splits);
-        if (!rc)
-        {
-            cudaError_t e = q->kt->lhe_combine_pair(c0, c1, key_a, key_b, n, stacked, stacked + elements,
-                                                    stacked + 2 * elements, 3 * elements, elements, !capturing(ctx),
-                                                    q->h, ctx->stream);
-            if (e != cudaSuccess)
-            {
-                return cuda_fail(e, "launching combine");
-            }
-            ++ctx->launches;
-        }
-        return rc;
+        return run_tc_encrypt(ctx, q, n, batch, parts, TcCombine{key_a, key_b, c0, c1}, ws, tc_splits);
     }
     return encrypt_cuda_cores(ctx, q, p, n, batch, key_a, key_b, coefficients, c0, c1, ws, nullptr, false);
 }

@@ -13,6 +13,7 @@
 #include "ntt.cuh"
 #include "pair.cuh"
 #include "plain.cuh"
+#include "tail.cuh"
 #include "tensor_ntt.cuh"
 
 namespace hmpc_gb300
@@ -106,6 +107,9 @@ namespace hmpc_gb300
         // (for the tensor-core engine, whose first group reads memory)
         cudaError_t (*uniform_pairs)(uint32_t* out, uint32_t log_n, uint64_t elements, const RngKey& rng,
                                      int words, uint32_t top_mask, const HostModulus& m, cudaStream_t stream);
+        // the last stages of a forward tensor-core transform (tail.cuh)
+        cudaError_t (*tc_tail)(const TailParams& p, bool encrypt, bool dependent, const HostModulus& m,
+                               cudaStream_t stream);
         // one pass of the one-butterfly-per-thread transform (pair.cuh)
         cudaError_t (*ntt_pair)(const PairPassParams& p, int kind, int nw, bool inverse, const HostModulus& m,
                                 unsigned grid, unsigned block, size_t smem, cudaStream_t stream);

@@ -45,6 +45,10 @@ namespace hmpc_gb300::detail
     struct TcTables
     {
         std::vector<TcGroupPlan> groups;
+        // forward, q of at least 32L - 14 bits: the last group's stages run as
+        // butterflies on the CUDA cores (tail.cuh) and have no constants here;
+        // the group before it leaves its values times 2^32
+        bool tail = false;
         uint8_t* images = nullptr;     // every group's constants (first group fed by limbs)
         size_t bytes = 0;
         uint8_t* first_cbd = nullptr;  // first group fed by centred binomial samples
@@ -292,15 +296,25 @@ namespace hmpc_gb300::detail
     // as p * sample + lift(m)) that share every constant past their first
     // group: one first-group launch per part into its slice of one digit
     // buffer, then the remaining groups once over count * batch polynomials.
-    // Part j draws with the context nonce advanced by j * n * batch; out holds
-    // the parts' results side by side (plane stride count * n * batch).
+    // Part j draws with the context nonce advanced by j * n * batch.
     struct TcStackPart
     {
         uint32_t vx2 = 0;
         const TcSmallInput* small = nullptr;  // nullptr: plain CBD(V) input
     };
-    int run_tc_stacked(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, const TcStackPart* parts,
-                       int count, uint32_t* out, int splits);
+    // BGV encryption from three stacked parts u, x, w: c0 = a * u + x and
+    // c1 = b * u + w in the last stages' kernel, or (tc_tail false) by a combine
+    // over `stacked`, 3 * n * batch * L words of workspace
+    struct TcCombine
+    {
+        const uint32_t* key_a;
+        const uint32_t* key_b;
+        uint32_t* c0;
+        uint32_t* c1;
+    };
+    bool tc_tail(const hmpc_modulus* mod, uint64_t n, bool inverse);
+    int run_tc_encrypt(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, const TcStackPart (&parts)[3],
+                       const TcCombine& combine, uint32_t* stacked, int splits);
     int tc_cost(hmpc_modulus* mod, uint64_t n, uint64_t batch, bool inverse, int kind, int splits, hmpc_tc_cost* out);
     // Polynomials of one degree n in buffers of their own (the batched
     // transform's buckets).  tc_prepare_polys builds the constants of (n,

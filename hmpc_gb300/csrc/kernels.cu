@@ -8,6 +8,7 @@
 #include "linalg.cuh"
 #include "ntt.cuh"
 #include "pair.cuh"
+#include "tail.cuh"
 
 #ifndef HMPC_L
 #error "compile with -DHMPC_L=<limbs>"
@@ -467,6 +468,15 @@ namespace hmpc_gb300
             return cudaGetLastError();
         }
 
+        cudaError_t tc_tail(const TailParams& p, bool encrypt, bool dependent, const HostModulus& h,
+                            cudaStream_t stream)
+        {
+            const unsigned grid = static_cast<unsigned>(((p.end - p.begin) / 2 + 255) / 256);
+            const Modulus<L> m = device_modulus(h);
+            return encrypt ? launch(tc_tail_kernel<L, true>, grid, 256, 0, dependent, stream, p, m)
+                           : launch(tc_tail_kernel<L, false>, grid, 256, 0, dependent, stream, p, m);
+        }
+
         cudaError_t ntt_cluster(const ClusterNttParams& p, uint64_t batch, const HostModulus& h, cudaStream_t stream)
         {
             if (batch == 0)
@@ -494,7 +504,7 @@ namespace hmpc_gb300
         const KernelTable table = {fma, binary, lhe_combine, uniform, cbd, to_montgomery,
                                    from_montgomery, cast, plain_stage, ct_mul, dec_combine, ntt_batched,
                                    ntt_batched_blocks_per_sm, lhe_combine_pair, lhe_key, matvec, matvec_monomial,
-                                   reduce, plane_sum, equal, ntt_cluster, uniform_pairs, ntt_pair};
+                                   reduce, plane_sum, equal, ntt_cluster, uniform_pairs, tc_tail, ntt_pair};
     }
 
     const KernelTable* HMPC_CAT(kernel_table_, HMPC_L)()

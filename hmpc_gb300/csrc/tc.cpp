@@ -21,7 +21,7 @@ namespace
     // groups of three stages from the first stage on; the remainder (1-3
     // stages) is the last group, whose constants are the most numerous in the
     // forward direction (one matrix per block above it)
-    std::vector<TcGroupPlan> plan_groups(const TcKernels* k, int log_n, bool inverse, int contiguous_splits)
+    std::vector<TcGroupPlan> plan_groups(const TcKernels* k, int log_n, bool inverse, int contiguous_splits, bool tail)
     {
         const int count = (log_n + 2) / 3;
         std::vector<TcGroupPlan> groups;
@@ -47,7 +47,7 @@ namespace
         // blocked per row (one contiguous run per row instead of a short piece
         // per word plane), written so by the group before it
         TcGroupPlan& last = groups.back();
-        if (last.lo == 0 && last.shape.splits == 1 && last.in_kind == tc_in_digits && groups.size() >= 2)
+        if (!tail && last.lo == 0 && last.shape.splits == 1 && last.in_kind == tc_in_digits && groups.size() >= 2)
         {
             last.layout |= 1;
             groups[groups.size() - 2].layout |= 2;
@@ -123,8 +123,9 @@ namespace
         ex.image_bytes = gp.shape.b_bytes;
         // the loaders of r = 8 groups fed by digits or limbs whose rows are
         // strided elements (the kernel's contiguous variant runs where lo = 0)
-        // take word-major K
-        ex.word_major = ex.r == 8 && d_in >= ex.dc && gp.lo != 0 ? 1u : 0u;
+        // take word-major K; the sampling loaders (whose nine small digits
+        // outnumber those of a two-limb modulus) do not
+        ex.word_major = !montgomery && ex.r == 8 && d_in >= ex.dc && gp.lo != 0 ? 1u : 0u;
         for (int j = 0; j < mod->c.limbs; ++j)
         {
             ex.half[j] = mod->c.half[static_cast<size_t>(j)];
@@ -144,8 +145,9 @@ namespace
         const int log_n = __builtin_ctzll(n);
         const TcKernels* k = kernels_of(mod);
         const int L = mod->c.limbs;
+        const bool tail = tc_tail(mod, n, inverse);
         std::lock_guard<std::mutex> lock(mod->tables_mutex);
-        auto key = std::make_tuple(log_n, inverse ? 1 : 0, splits);
+        auto key = std::make_tuple(log_n, inverse ? 1 : 0, tail ? 1 : splits);
         auto it = mod->tc_tables.find(key);
         const bool fresh = it == mod->tc_tables.end();
         if (!fresh && !it->second.fit)
@@ -165,18 +167,25 @@ namespace
         }
         else
         {
-            tt.groups = plan_groups(k, log_n, inverse, splits);
+            tt.groups = plan_groups(k, log_n, inverse, splits, tail);
+            tt.tail = tail;
             size_t bytes = 0;
-            for (auto& gp : tt.groups)
+            for (size_t i = 0; i + (tail ? 1 : 0) < tt.groups.size(); ++i)
             {
+                TcGroupPlan& gp = tt.groups[i];
                 gp.offset = bytes;
                 bytes += static_cast<size_t>(gp.blocks) * gp.shape.splits * gp.shape.b_bytes;
                 bytes = (bytes + 255) & ~static_cast<size_t>(255);
             }
             tt.bytes = bytes;
         }
-        // 256^a * R mod q for every digit slot
-        const uint32_t slots = static_cast<uint32_t>(k->digits + 2);
+        // 256^a * R mod q for every digit slot, and four more: the constants of
+        // the group before the tail are those of a + 4 (times 2^32)
+        const uint32_t slots = static_cast<uint32_t>(k->digits + 2 + 4);
+        const size_t constant_groups = tt.groups.size() - (tail ? 1 : 0);
+        auto digit_powers = [&](const uint32_t* pow, size_t group) {
+            return pow + (tail && group + 1 == constant_groups ? 4u * static_cast<uint32_t>(L) : 0u);
+        };
         std::vector<uint32_t> pow256(static_cast<size_t>(slots) * L);
         for (uint32_t a = 0; a < slots; ++a)
         {
@@ -189,8 +198,9 @@ namespace
             }
         }
         uint64_t gx_words = 0;
-        for (const auto& gp : tt.groups)
+        for (size_t i = 0; i < constant_groups; ++i)
         {
+            const TcGroupPlan& gp = tt.groups[i];
             gx_words = std::max<uint64_t>(gx_words, (gp.blocks << (2 * gp.g)) * static_cast<uint64_t>(L));
         }
         uint32_t* d_pow = nullptr;
@@ -220,10 +230,11 @@ namespace
                 return fail(HMPC_ERROR_OUT_OF_MEMORY, "allocating tensor-core constants");
             }
             cudaMemsetAsync(tt.images, 0, tt.bytes, ctx->stream);
-            for (const auto& gp : tt.groups)
+            for (size_t i = 0; i < constant_groups; ++i)
             {
+                const TcGroupPlan& gp = tt.groups[i];
                 if (int rc = build_group(ctx, mod, t, log_n, inverse, gp, false, gp.shape.d_in, tt.images + gp.offset,
-                                         d_gx, d_pow))
+                                         d_gx, digit_powers(d_pow, i)))
                 {
                     cleanup();
                     cudaFree(tt.images);
@@ -462,6 +473,13 @@ namespace hmpc_gb300::detail
         return mod->c.q[static_cast<size_t>(L - 1)] >= 32u;
     }
 
+    bool tc_tail(const hmpc_modulus* mod, uint64_t n, bool inverse)
+    {
+        // the one-row reduction of the tail's inputs needs 2^(32L + 17) <= 2^32 q,
+        // and the group before the tail is one fed by digits (three groups)
+        return !inverse && n > 64 && mod->c.bits >= 32 * mod->c.limbs - 14;
+    }
+
     bool tc_applicable(const hmpc_modulus* mod, int log_n, int kind, const uint32_t* poly_rng)
     {
         return log_n >= 4 && !poly_rng && (kind == producer_tensor || kind == producer_cbd || kind == producer_uniform) &&
@@ -584,6 +602,94 @@ namespace hmpc_gb300::detail
             return HMPC_OK;
         }
 
+        // the stages of the last group on the CUDA cores: `elements` of each part
+        // from digit planes of plane stride `stride` into limb planes at `out`
+        // (or out_polys), or the parts combined into a ciphertext
+        int tail(const uint32_t* in, uint32_t* out, uint64_t stride, uint64_t elements, const TcCombine* combine)
+        {
+            Tables* t = nullptr;
+            if (int rc = mod->prepare(1ull << log_n, &t))
+            {
+                return rc;
+            }
+            const int L = mod->c.limbs;
+            TailParams p{};
+            p.digits = in;
+            p.stride = stride;
+            p.elements = elements;
+            p.twiddles = t->forward;
+            p.log_n = log_n;
+            p.w = tt->groups.back().g;
+            p.out = out;
+            p.out_polys = out_polys;
+            if (combine)
+            {
+                p.key_a = combine->key_a;
+                p.key_b = combine->key_b;
+                p.c0 = combine->c0;
+                p.c1 = combine->c1;
+            }
+            // the multiple of q nearest above 2^(32L + 16), less 128 for each digit
+            host::words c(static_cast<size_t>(L + 1), 0u);
+            c[static_cast<size_t>(L)] = 1u << 16;
+            c = host::resize(host::sub(c, host::mod(c, mod->c.q), L + 2), L + 2);
+            uint64_t carry = 0;
+            for (int j = 0; j < L; ++j)
+            {
+                carry += static_cast<uint64_t>(c[static_cast<size_t>(j)]) + mod->c.q[static_cast<size_t>(j)];
+                c[static_cast<size_t>(j)] = static_cast<uint32_t>(carry);
+                carry >>= 32;
+            }
+            c[static_cast<size_t>(L)] += static_cast<uint32_t>(carry);
+            int64_t borrow = 0;
+            for (int j = 0; j <= L; ++j)
+            {
+                const int64_t d = static_cast<int64_t>(c[static_cast<size_t>(j)]) - 0x80808080ll + borrow;
+                p.offset[j] = static_cast<uint32_t>(d);
+                borrow = d >> 32;
+            }
+            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+            const bool dependent = cudaStreamIsCapturing(stream, &capture) == cudaSuccess &&
+                                   capture == cudaStreamCaptureStatusNone;
+            // an encryption in two launches, either half of its coefficients: it
+            // keeps its number of launches (one per group and a combination)
+            const int launches = combine ? 2 : 1;
+            for (int i = 0; i < launches; ++i)
+            {
+                p.begin = static_cast<uint64_t>(i) * (elements / static_cast<uint64_t>(launches));
+                p.end = p.begin + elements / static_cast<uint64_t>(launches);
+                cudaError_t e = mod->kt->tc_tail(p, combine != nullptr, dependent, mod->h, stream);
+                if (e != cudaSuccess)
+                {
+                    return cuda_fail(e, "launching the last stages");
+                }
+                ++ctx->launches;
+            }
+            return HMPC_OK;
+        }
+
+        // groups first..last of a plan over `batch` polynomials in digit planes of
+        // stride `elements`, the two digit buffers taking turns
+        int groups(size_t first, uint32_t* digits, uint32_t* out, uint64_t elements, uint64_t batch,
+                   const TcCombine* combine, uint64_t part_elements, bool dependent = true)
+        {
+            const uint64_t w = tt->groups.front().shape.w_out;
+            const size_t stages = tt->groups.size();
+            for (size_t j = first; j < stages; ++j)
+            {
+                const uint32_t* in = digits + (((j - 1) & 1u) ? w * elements : 0);
+                uint32_t* o = j + 1 == stages ? out : digits + ((j & 1u) ? w * elements : 0);
+                const int rc = j + 1 == stages && tt->tail
+                                   ? tail(in, o, elements, part_elements, combine)
+                                   : group(j, in, o, elements, batch, tc_in_digits, 0, nullptr, elements, dependent);
+                if (rc)
+                {
+                    return rc;
+                }
+            }
+            return HMPC_OK;
+        }
+
         // the first six stages of `batch` CBD(vx2)-fed transforms in one wide
         // group (images: the eight images of G6 or G6 * p), written as digit
         // planes of plane stride `stride` at `out`
@@ -673,28 +779,22 @@ namespace hmpc_gb300::detail
             {
                 return rc;
             }
-            for (size_t j = 2; j < stages; ++j)
+            if (int rc = run.groups(2, digits, out, elements, batch, nullptr, elements))
             {
-                const uint32_t* in = digits + (((j - 1) & 1u) ? w * elements : 0);
-                uint32_t* o = j + 1 == stages ? out : digits + ((j & 1u) ? w * elements : 0);
-                if (int rc = run.group(j, in, o, elements, batch, tc_in_digits, 0, nullptr, elements, true))
-                {
-                    return rc;
-                }
+                return rc;
             }
             nonce_add(ctx->nonce, elements);
             return HMPC_OK;
         }
         const int first_kind = cbd ? (small ? tc_in_small : tc_in_cbd) : tc_in_limbs;
-        for (size_t j = 0; j < stages; ++j)
+        int rc = run.group(0, src, stages == 1 ? out : digits, elements, batch, first_kind, vx2, small, elements);
+        if (!rc)
         {
-            const uint32_t* in = j == 0 ? src : digits + (((j - 1) & 1u) ? w * elements : 0);
-            uint32_t* o = j + 1 == stages ? out : digits + ((j & 1u) ? w * elements : 0);
-            if (int rc = run.group(j, in, o, elements, batch, j == 0 ? first_kind : tc_in_digits, vx2,
-                                   j == 0 ? small : nullptr, elements, j > 0))
-            {
-                return rc;
-            }
+            rc = run.groups(1, digits, out, elements, batch, nullptr, elements);
+        }
+        if (rc)
+        {
+            return rc;
         }
         if (cbd)
         {
@@ -703,9 +803,10 @@ namespace hmpc_gb300::detail
         return HMPC_OK;
     }
 
-    int run_tc_stacked(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, const TcStackPart* parts,
-                       int count, uint32_t* out, int splits)
+    int run_tc_encrypt(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, const TcStackPart (&parts)[3],
+                       const TcCombine& combine, uint32_t* stacked, int splits)
     {
+        constexpr int count = 3;
         bool need_cbd = false, need_small = false;
         for (int i = 0; i < count; ++i)
         {
@@ -793,42 +894,43 @@ namespace hmpc_gb300::detail
                     return rc;
                 }
             }
-            for (size_t j = 2; j < stages; ++j)
+            if (int rc = run.groups(2, digits, stacked, total, batch * count, &combine, elements))
             {
-                const uint32_t* in = digits + (((j - 1) & 1u) ? w * total : 0);
-                uint32_t* o = j + 1 == stages ? out : digits + ((j & 1u) ? w * total : 0);
-                if (int rc = run.group(j, in, o, total, batch * static_cast<uint64_t>(count), tc_in_digits, 0, nullptr,
-                                       0, true))
+                return rc;
+            }
+        }
+        else
+        {
+            // first groups: part i into its slice of buffer 0 (plane-major slices,
+            // or whole blocked runs when the next group is the last)
+            const bool blocked = (tt->groups.front().layout & 2) != 0;
+            for (int i = 0; i < count; ++i)
+            {
+                uint32_t* slice = digits + static_cast<uint64_t>(i) * elements * (blocked ? w : 1);
+                const int kind = parts[i].small ? tc_in_small : tc_in_cbd;
+                if (int rc = run.group(0, nullptr, stages == 1 ? stacked + static_cast<uint64_t>(i) * elements : slice,
+                                       total, batch, kind, parts[i].vx2, parts[i].small, elements, i > 0))
                 {
                     return rc;
                 }
+                nonce_add(ctx->nonce, elements);
             }
-            return HMPC_OK;
-        }
-        // first groups: part i into its slice of buffer 0 (plane-major slices,
-        // or whole blocked runs when the next group is the last)
-        const bool blocked = (tt->groups.front().layout & 2) != 0;
-        for (int i = 0; i < count; ++i)
-        {
-            uint32_t* slice = digits + static_cast<uint64_t>(i) * elements * (blocked ? w : 1);
-            const int kind = parts[i].small ? tc_in_small : tc_in_cbd;
-            if (int rc = run.group(0, nullptr, stages == 1 ? out + static_cast<uint64_t>(i) * elements : slice, total,
-                                   batch, kind, parts[i].vx2, parts[i].small, elements, i > 0))
+            // the shared groups over the stacked batch
+            if (int rc = run.groups(1, digits, stacked, total, batch * count, &combine, elements))
             {
                 return rc;
             }
-            nonce_add(ctx->nonce, elements);
         }
-        // the shared groups over the stacked batch
-        for (size_t j = 1; j < stages; ++j)
+        if (!tt->tail)
         {
-            const uint32_t* in = digits + (((j - 1) & 1u) ? w * total : 0);
-            uint32_t* o = j + 1 == stages ? out : digits + ((j & 1u) ? w * total : 0);
-            if (int rc = run.group(j, in, o, total, batch * static_cast<uint64_t>(count), tc_in_digits, 0, nullptr, 0,
-                                   true))
+            cudaError_t e = mod->kt->lhe_combine_pair(combine.c0, combine.c1, combine.key_a, combine.key_b, n, stacked,
+                                                      stacked + elements, stacked + 2 * elements, total, elements,
+                                                      !capturing(ctx), mod->h, ctx->stream);
+            if (e != cudaSuccess)
             {
-                return rc;
+                return cuda_fail(e, "launching combine");
             }
+            ++ctx->launches;
         }
         return HMPC_OK;
     }
@@ -862,7 +964,8 @@ namespace hmpc_gb300::detail
         TcTables* tt = nullptr;
         {
             std::lock_guard<std::mutex> lock(mod->tables_mutex);
-            auto it = mod->tc_tables.find(std::make_tuple(__builtin_ctzll(n), inverse ? 1 : 0, splits));
+            auto it = mod->tc_tables.find(
+                std::make_tuple(__builtin_ctzll(n), inverse ? 1 : 0, tc_tail(mod, n, inverse) ? 1 : splits));
             if (it == mod->tc_tables.end() || !it->second.fit || !it->second.images)
             {
                 return fail(HMPC_ERROR_INVALID_ARGUMENT, "tensor-core constants not prepared for this degree");
@@ -870,8 +973,6 @@ namespace hmpc_gb300::detail
             tt = &it->second;
         }
         const uint64_t elements = n * count;
-        const uint64_t w = tt->groups.front().shape.w_out;
-        const size_t stages = tt->groups.size();
         TcLaunch run;
         if (int rc = run.init(ctx, mod, n, tt))
         {
@@ -880,16 +981,12 @@ namespace hmpc_gb300::detail
         run.stream = stream;
         run.in_polys = in_polys;
         run.out_polys = out_polys;
-        for (size_t j = 0; j < stages; ++j)
+        if (int rc = run.group(0, nullptr, tt->groups.size() == 1 ? nullptr : digits, elements, count, tc_in_limbs, 0,
+                               nullptr, 0))
         {
-            const uint32_t* in = j == 0 ? nullptr : digits + (((j - 1) & 1u) ? w * elements : 0);
-            uint32_t* o = j + 1 == stages ? nullptr : digits + ((j & 1u) ? w * elements : 0);
-            if (int rc = run.group(j, in, o, elements, count, j == 0 ? tc_in_limbs : tc_in_digits, 0, nullptr, 0))
-            {
-                return rc;
-            }
+            return rc;
         }
-        return HMPC_OK;
+        return run.groups(1, digits, nullptr, elements, count, nullptr, elements, false);
     }
 
     int tc_cost(hmpc_modulus* mod, uint64_t n, uint64_t batch, bool inverse, int kind, int splits, hmpc_tc_cost* out)
@@ -901,7 +998,8 @@ namespace hmpc_gb300::detail
         }
         const TcKernels* k = kernels_of(mod);
         const int log_n = __builtin_ctzll(n);
-        const std::vector<TcGroupPlan> groups = plan_groups(k, log_n, inverse, splits);
+        const bool tail = tc_tail(mod, n, inverse);
+        const std::vector<TcGroupPlan> groups = plan_groups(k, log_n, inverse, splits, tail);
         const double elements = static_cast<double>(n) * static_cast<double>(batch);
         const double limb_bytes = 4.0 * mod->c.limbs;
         out->launches = static_cast<uint32_t>(groups.size());
@@ -923,6 +1021,12 @@ namespace hmpc_gb300::detail
         for (size_t j = first; j < groups.size(); ++j)
         {
             TcShapeInfo shape = groups[j].shape;
+            if (tail && j + 1 == groups.size())
+            {
+                // no constants and no MMAs: digit planes in, limb planes out
+                out->bytes += elements * (4.0 * groups[j - 1].shape.w_out + limb_bytes);
+                continue;
+            }
             const bool cbd = j == 0 && kind == producer_cbd;
             if (cbd)
             {
@@ -956,7 +1060,8 @@ namespace hmpc_gb300::detail
             return rc;
         }
         std::lock_guard<std::mutex> lock(mod->tables_mutex);
-        auto it = mod->tc_tables.find(std::make_tuple(__builtin_ctzll(n), inverse ? 1 : 0, splits));
+        auto it = mod->tc_tables.find(
+            std::make_tuple(__builtin_ctzll(n), inverse ? 1 : 0, tc_tail(mod, n, inverse) ? 1 : splits));
         if (it == mod->tc_tables.end())
         {
             return rc ? rc : fail(HMPC_ERROR_CUDA, "tensor-core constants missing");
