@@ -53,7 +53,7 @@ namespace hmpc_gb300
     // Bound by the wide multiply-adds: 1.5 products per element at w = 3, and
     // two more per ciphertext coefficient.  TAIL_FIGURES
     template<int L, bool Encrypt>
-    __global__ void __launch_bounds__(256) tc_tail_kernel(const TailParams p, const Modulus<L> m)
+    __global__ void __launch_bounds__(256, 3) tc_tail_kernel(const TailParams p, const Modulus<L> m)
     {
         const uint32_t w = p.w;
         const uint64_t id = p.begin / 2 + static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
