@@ -1,12 +1,12 @@
 // The last stages of a forward tensor-core transform, on the CUDA cores.
 //
-// The last group of stages works on adjacent elements: on the tensor cores it
-// has one constant matrix per 2^w elements (0.57 GB for 2^15 coefficients at
-// 8 limbs), a digit tile and an epilogue per matrix, and fills an SM's shared
-// memory with one CTA whose nine warps wait on one another: 325 us for 256
-// polynomials, a third of its HBM rate.  As butterflies the same stages need
-// 1.5 products per element at w = 3, on a pipe the tensor-core groups leave
-// idle.
+// On the tensor cores a group of stages with few index bits below it has one
+// constant matrix per few elements (0.57 GB for the last three stages of 2^15
+// coefficients at 8 limbs), a digit tile and an epilogue per matrix, and fills an
+// SM's shared memory with one CTA whose nine warps wait on one another: 1001 us
+// for 768 polynomials, a third of its HBM rate.  As butterflies the last w
+// stages need w / 2 products per element, on a pipe the tensor-core groups
+// leave idle.
 //
 // The groups before leave each value as biased base-256 digits of an integer
 // congruent to the residue times 2^32 (the factor is in the constants of the
@@ -50,8 +50,11 @@ namespace hmpc_gb300
         uint32_t* c1;
     };
 
-    // Bound by the wide multiply-adds: 1.5 products per element at w = 3, and
-    // two more per ciphertext coefficient.  TAIL_FIGURES
+    // Bound by the wide multiply-adds (their pipe 70 % busy): 1.5 products per
+    // element at w = 3, and two more per ciphertext coefficient.  256 encryptions
+    // of 2^15 at 8 limbs: 1072 us, against 1001 for the group on the tensor cores
+    // and 355 for the combination after it.  Three blocks per SM (80 registers, a
+    // few spills): 1118 us at two blocks, 1075 at four.
     template<int L, bool Encrypt>
     __global__ void __launch_bounds__(256, 3) tc_tail_kernel(const TailParams p, const Modulus<L> m)
     {

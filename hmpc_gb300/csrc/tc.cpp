@@ -18,12 +18,25 @@ namespace
         return tc_kernels(mod->c.limbs);
     }
 
+    // launches of a transform's groups of up to three stages; a transform with a
+    // tail keeps the number (the tail takes the launches of the groups it
+    // replaces, a share of the elements each)
+    int group_launches(int log_n)
+    {
+        return (log_n + 2) / 3;
+    }
+
     // groups of three stages from the first stage on; the remainder (1-3
     // stages) is the last group, whose constants are the most numerous in the
-    // forward direction (one matrix per block above it)
+    // forward direction (one matrix per block above it).  With a tail the
+    // remainder is its 3 to 5 stages: a tensor-core group needs a constant matrix
+    // per 8 * 2^lo elements, lo the index bits below it, so at lo of 1 or 2 the
+    // constants outweigh the data (2^16, 6 limbs, 103 polynomials: stages 12-14 as
+    // a group and the last one as tail 295 + 72 us; the batch of 512 polynomials
+    // of 2^12..2^16 this is part of: 1174 us so, 961 with all four as tail).
     std::vector<TcGroupPlan> plan_groups(const TcKernels* k, int log_n, bool inverse, int contiguous_splits, bool tail)
     {
-        const int count = (log_n + 2) / 3;
+        const int count = tail ? (log_n - 3) / 3 + 1 : group_launches(log_n);
         std::vector<TcGroupPlan> groups;
         for (int j = 0; j < count; ++j)
         {
@@ -315,16 +328,16 @@ namespace
 
     // whether a forward plan starts with two three-stage groups and has at
     // least two more after them (the wide group replaces the first two)
-    bool wide_plan(const std::vector<TcGroupPlan>& groups)
+    bool wide_plan(const std::vector<TcGroupPlan>& groups, bool tail)
     {
         // the second group must write plain planes (not the blocked runs of a
         // group before the last)
-        return groups.size() >= 4 && groups[0].g == 3 && groups[1].g == 3 && (groups[1].layout & 2) == 0;
+        return groups.size() >= (tail ? 3u : 4u) && groups[0].g == 3 && groups[1].g == 3 && (groups[1].layout & 2) == 0;
     }
 
     bool wide_plan(const TcTables* tt)
     {
-        return wide_plan(tt->groups);
+        return wide_plan(tt->groups, tt->tail);
     }
 
     // the wide group's images: unscaled, and scaled by p (nullptr: not needed)
@@ -390,8 +403,9 @@ namespace
                 return cuda_fail(e, "generating tensor-core constants");
             }
         }
-        // raw samples: one digit slot, 256^0 * R
-        const host::words one = host::to_mont(mod->c, host::words{1u});
+        // raw samples: one digit slot, 256^0 * R (times 2^32 right before the tail)
+        const host::words one = host::to_mont(
+            mod->c, tt->tail && tt->groups.size() == 3 ? host::words{0u, 1u} : host::words{1u});
         cudaMemcpyAsync(d_pow, one.data(), L * sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream);
         for (int variant = 0; variant < 2; ++variant)
         {
@@ -476,8 +490,8 @@ namespace hmpc_gb300::detail
     bool tc_tail(const hmpc_modulus* mod, uint64_t n, bool inverse)
     {
         // the one-row reduction of the tail's inputs needs 2^(32L + 17) <= 2^32 q,
-        // and the group before the tail is one fed by digits (three groups)
-        return !inverse && n > 64 && mod->c.bits >= 32 * mod->c.limbs - 14;
+        // and the group before the tail is one fed by digits (two groups)
+        return !inverse && n >= 512 && mod->c.bits >= 32 * mod->c.limbs - 14;
     }
 
     bool tc_applicable(const hmpc_modulus* mod, int log_n, int kind, const uint32_t* poly_rng)
@@ -651,13 +665,17 @@ namespace hmpc_gb300::detail
             cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
             const bool dependent = cudaStreamIsCapturing(stream, &capture) == cudaSuccess &&
                                    capture == cudaStreamCaptureStatusNone;
-            // an encryption in two launches, either half of its coefficients: it
-            // keeps its number of launches (one per group and a combination)
-            const int launches = combine ? 2 : 1;
-            for (int i = 0; i < launches; ++i)
+            // the launches of the groups it replaces, and of an encryption's
+            // combination (one for polynomials in buffers of their own)
+            const uint64_t launches =
+                out_polys ? 1
+                          : static_cast<uint64_t>(group_launches(static_cast<int>(log_n))) - (tt->groups.size() - 1) +
+                                (combine ? 1 : 0);
+            const uint64_t tiles = elements >> p.w;
+            for (uint64_t i = 0; i < launches; ++i)
             {
-                p.begin = static_cast<uint64_t>(i) * (elements / static_cast<uint64_t>(launches));
-                p.end = p.begin + elements / static_cast<uint64_t>(launches);
+                p.begin = i * tiles / launches << p.w;
+                p.end = (i + 1) * tiles / launches << p.w;
                 cudaError_t e = mod->kt->tc_tail(p, combine != nullptr, dependent, mod->h, stream);
                 if (e != cudaSuccess)
                 {
@@ -1002,11 +1020,11 @@ namespace hmpc_gb300::detail
         const std::vector<TcGroupPlan> groups = plan_groups(k, log_n, inverse, splits, tail);
         const double elements = static_cast<double>(n) * static_cast<double>(batch);
         const double limb_bytes = 4.0 * mod->c.limbs;
-        out->launches = static_cast<uint32_t>(groups.size());
+        out->launches = static_cast<uint32_t>(group_launches(log_n));
         out->bytes = 0.0;
         out->flops = 0.0;
         size_t first = 0;
-        if (kind == producer_cbd && wide_plan(groups))
+        if (kind == producer_cbd && wide_plan(groups, tail))
         {
             // the wide group: digit planes written, eight images read, eight
             // N = 256 products of K = 64 per 128-row tile

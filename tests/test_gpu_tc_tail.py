@@ -1,5 +1,5 @@
 """The tensor-core forward transform's last stages on the CUDA cores: every
-number of stages they can be (1 to 3), the smallest modulus that takes them and
+number of stages they can be (3 to 5), the smallest modulus that takes them and
 the largest that does not, odd batches that leave the last block unfilled,
 largest inputs, plain and as an encryption -- against the oracle."""
 import numpy as np
@@ -16,11 +16,11 @@ KEY = [3, 1, 4, 1, 5, 9, 2, 6]
 
 @pytest.mark.parametrize("limbs", range(2, 9))
 @pytest.mark.parametrize("short", [0, 14, 15])
-@pytest.mark.parametrize("log_n,batch", [(6, 9), (7, 1), (7, 3), (8, 2), (10, 5), (11, 3), (12, 1)])
+@pytest.mark.parametrize("log_n,batch", [(8, 5), (9, 1), (9, 3), (10, 5), (11, 3), (12, 1), (13, 2), (14, 1)])
 def test_tail(oracle, cpu_threads, limbs, short, log_n, batch):
     n = 1 << log_n
     # one bit below a full top byte where the digits of q / 2 would overflow
-    q_value = _prime(32 * limbs - short, 1 << 13) if short else _prime(32 * limbs - 1, 1 << 13)
+    q_value = _prime(32 * limbs - (short or 1), 1 << 15)
     queue = Queue(key=KEY)
     q, oq = queue.modulus(q_value), oracle.Modulus(q_value)
     q.set_plan(n, batch, False, radix_bits=0)
