@@ -348,7 +348,7 @@ namespace hmpc_gb300
     }
 
     template<int L, int Kind, int NW, bool Inverse>
-    __global__ void __launch_bounds__(pair_max_threads) ntt_pair_kernel(const PairPassParams p, const Modulus<L> m)
+    __global__ void __launch_bounds__(pair_max_threads, 2) ntt_pair_kernel(const PairPassParams p, const Modulus<L> m)
     {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         extern __shared__ uint32_t exchange[];
@@ -394,7 +394,7 @@ namespace hmpc_gb300
     }
 
     template<int L, bool Inverse>
-    __global__ void __launch_bounds__(pair_max_threads) ntt_batched_kernel(const BatchedParams bp, const Modulus<L> m)
+    __global__ void __launch_bounds__(pair_max_threads, 2) ntt_batched_kernel(const BatchedParams bp, const Modulus<L> m)
     {
         extern __shared__ uint32_t exchange[];
         __shared__ uint32_t item_s;
