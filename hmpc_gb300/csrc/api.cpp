@@ -143,15 +143,7 @@ namespace hmpc_gb300::detail
             return fail(HMPC_ERROR_INVALID_ARGUMENT, "tensor producer without source");
         }
         const int log_n = __builtin_ctzll(n);
-        hmpc_modulus::TileChoice choice;
-        {
-            std::lock_guard<std::mutex> lock(mod->tables_mutex);
-            auto it = mod->tile_choices.find(std::make_tuple(log_n, inverse ? 1 : 0, batch));
-            if (it != mod->tile_choices.end())
-            {
-                choice = it->second;
-            }
-        }
+        hmpc_modulus::TileChoice choice = mod->choice(n, inverse, batch);
         if (choice.radix_bits == 0)
         {
             // tensor-core engine; calls it does not cover run the default CUDA-core tiles
@@ -292,6 +284,48 @@ namespace hmpc_gb300::detail
 
 namespace hmpc_gb300::detail
 {
+    bool overlap(const uint32_t* a, uint64_t a_words, const uint32_t* b, uint64_t b_words)
+    {
+        return a < b + b_words && b < a + a_words;
+    }
+
+    // the lift of INTT_q(c0 - s*c1) to p in the inverse transform's own passes
+    int run_decrypt(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n, uint64_t batch, const uint32_t* s,
+                    const uint32_t* c0, const uint32_t* c1, uint32_t* x, uint32_t* out,
+                    const std::vector<PairPlan>& plan)
+    {
+        Tables* t = nullptr;
+        if (int rc = q->prepare(n, &t))
+        {
+            return rc;
+        }
+        DecryptParams d{};
+        d.s = s;
+        d.c0 = c0;
+        d.c1 = c1;
+        d.out = out;
+        d.cast = make_cast(p, q);
+        std::copy(p->h.q, p->h.q + p->c.limbs, d.p);
+        d.pninv = p->h.ninv;
+        const bool dependent = !capturing(ctx);
+        for (size_t i = 0; i < plan.size(); ++i)
+        {
+            PairPassParams pp = plan[i].params;
+            pp.out[0] = x;
+            pp.twiddles = t->inverse;
+            pp.elements = n * batch;
+            pp.dependent = dependent ? 1u : 0u;
+            const cudaError_t e = q->kt->ntt_decrypt(pp, d, i == 0, i + 1 == plan.size() ? p->c.limbs : 0, q->h,
+                                                     plan[i].grid, plan[i].block, plan[i].smem, ctx->stream);
+            if (e != cudaSuccess)
+            {
+                return cuda_fail(e, "launching decryption pass");
+            }
+            ++ctx->launches;
+        }
+        return HMPC_OK;
+    }
+
     // x = c0 - s*c1 (+ s^2*c2) -> INTT_q -> cast to p (-> NTT_p)
     int decrypt(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n, uint64_t batch, const uint32_t* s,
                 const uint32_t* c0, const uint32_t* c1, const uint32_t* c2, int plaintext_ntt, uint32_t* out)
@@ -317,6 +351,26 @@ namespace hmpc_gb300::detail
         if (!x)
         {
             return fail(HMPC_ERROR_OUT_OF_MEMORY, "allocating the decryption workspace");
+        }
+        const hmpc_modulus::TileChoice choice = q->choice(n, true, batch);
+        if (!c2 && choice.radix_bits >= 2 && p->c.limbs <= 2 && host::compare(q->c.q, p->c.q) > 0)
+        {
+            const std::vector<PairPlan> plan =
+                plan_pairs(q->c.limbs, __builtin_ctzll(n), batch, true, choice.local_bits, choice.col_bits);
+            const uint64_t q_words = elements * static_cast<uint64_t>(q->c.limbs);
+            const uint64_t s_words = n * static_cast<uint64_t>(q->c.limbs);
+            const uint64_t out_words = elements * static_cast<uint64_t>(p->c.limbs);
+            // one pass that reads and writes: not over its own operands
+            if (plan.size() > 1 || !(overlap(out, out_words, c0, q_words) || overlap(out, out_words, c1, q_words) ||
+                                     overlap(out, out_words, s, s_words)))
+            {
+                if (int rc = run_decrypt(ctx, q, p, n, batch, s, c0, c1, x, out, plan))
+                {
+                    return rc;
+                }
+                return plaintext_ntt ? run_transform(ctx, p, n, batch, false, producer_tensor, 0, 0, out, out)
+                                     : HMPC_OK;
+            }
         }
         cudaError_t e = q->kt->dec_combine(x, s, n, c0, c1, c2, elements, q->h, ctx->stream);
         if (e != cudaSuccess)
@@ -791,15 +845,7 @@ int hmpc_modulus_get_plan(hmpc_modulus* mod, uint64_t n, uint64_t batch, int inv
     {
         return rc;
     }
-    hmpc_modulus::TileChoice choice;
-    {
-        std::lock_guard<std::mutex> lock(mod->tables_mutex);
-        auto it = mod->tile_choices.find(std::make_tuple(__builtin_ctzll(n), inverse ? 1 : 0, batch));
-        if (it != mod->tile_choices.end())
-        {
-            choice = it->second;
-        }
-    }
+    const hmpc_modulus::TileChoice choice = mod->choice(n, inverse != 0, batch);
     *radix_bits = choice.radix_bits;
     *local_bits = choice.local_bits;
     *col_bits = choice.col_bits;

@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 
+#include "cast.cuh"
 #include "chacha.cuh"
 #include "cluster.cuh"
 #include "linalg.cuh"
@@ -18,7 +19,6 @@
 
 namespace hmpc_gb300
 {
-    constexpr int max_device_limbs = 9;
     constexpr int max_wide_words = 2 * max_device_limbs + 2;
 
     struct HostModulus
@@ -30,19 +30,6 @@ namespace hmpc_gb300
         uint32_t one[16] = {};
         uint32_t r2[16] = {};
         uint32_t half[16] = {};
-    };
-
-    // constants of a centred lift from a source modulus into the target one
-    // (hmpc/ints/mod.hpp:259-307)
-    struct CastParams
-    {
-        uint32_t src_limbs;
-        uint32_t src_ninv;
-        uint32_t src_q[max_device_limbs];
-        uint32_t src_half[max_device_limbs];
-        uint32_t offset[max_device_limbs + 1];  // added when the value exceeds src/2
-        uint32_t direct;                          // 1: value + offset < target Q
-        uint32_t factor[max_device_limbs];        // R^2 (direct) or R'*R^2 mod Q
     };
 
     struct KernelTable
@@ -107,6 +94,11 @@ namespace hmpc_gb300
         // (for the tensor-core engine, whose first group reads memory)
         cudaError_t (*uniform_pairs)(uint32_t* out, uint32_t log_n, uint64_t elements, const RngKey& rng,
                                      int words, uint32_t top_mask, const HostModulus& m, cudaStream_t stream);
+        // one pass of a decryption's inverse transform; p_limbs: 1 or 2 in the
+        // last pass, else 0
+        cudaError_t (*ntt_decrypt)(const PairPassParams& p, const DecryptParams& d, bool first, int p_limbs,
+                                   const HostModulus& m, unsigned grid, unsigned block, size_t smem,
+                                   cudaStream_t stream);
         // the last stages of a forward tensor-core transform (tail.cuh)
         cudaError_t (*tc_tail)(const TailParams& p, bool encrypt, bool dependent, const HostModulus& m,
                                cudaStream_t stream);

@@ -219,6 +219,13 @@ struct hmpc_modulus
         int col_bits = 4;
     };
     std::map<std::tuple<int, int, uint64_t>, TileChoice> tile_choices;
+    // the shape set or tuned for these transforms, else the default
+    TileChoice choice(uint64_t n, bool inverse, uint64_t batch)
+    {
+        std::lock_guard<std::mutex> lock(tables_mutex);
+        auto it = tile_choices.find(std::make_tuple(__builtin_ctzll(n), inverse ? 1 : 0, batch));
+        return it != tile_choices.end() ? it->second : TileChoice{};
+    }
     std::mutex tables_mutex;  // the serving thread looks tables up while clients register new degrees
 
     // whether the twiddle tables of degree n exist (no allocation)

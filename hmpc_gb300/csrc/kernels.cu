@@ -468,6 +468,21 @@ namespace hmpc_gb300
             return cudaGetLastError();
         }
 
+        cudaError_t ntt_decrypt(const PairPassParams& p, const DecryptParams& d, bool first, int p_limbs,
+                                const HostModulus& h, unsigned grid, unsigned block, size_t smem, cudaStream_t stream)
+        {
+            const Modulus<L> m = device_modulus(h);
+            void (*kernel)(PairPassParams, DecryptParams, Modulus<L>) = nullptr;
+            switch (p_limbs)
+            {
+            case 0: kernel = first ? ntt_decrypt_kernel<L, true, 0> : ntt_decrypt_kernel<L, false, 0>; break;
+            case 1: kernel = first ? ntt_decrypt_kernel<L, true, 1> : ntt_decrypt_kernel<L, false, 1>; break;
+            case 2: kernel = first ? ntt_decrypt_kernel<L, true, 2> : ntt_decrypt_kernel<L, false, 2>; break;
+            default: return cudaErrorInvalidValue;
+            }
+            return launch(kernel, grid, block, smem, p.dependent != 0, stream, p, d, m);
+        }
+
         cudaError_t tc_tail(const TailParams& p, bool encrypt, bool dependent, const HostModulus& h,
                             cudaStream_t stream)
         {
@@ -504,7 +519,7 @@ namespace hmpc_gb300
         const KernelTable table = {fma, binary, lhe_combine, uniform, cbd, to_montgomery,
                                    from_montgomery, cast, plain_stage, ct_mul, dec_combine, ntt_batched,
                                    ntt_batched_blocks_per_sm, lhe_combine_pair, lhe_key, matvec, matvec_monomial,
-                                   reduce, plane_sum, equal, ntt_cluster, uniform_pairs, tc_tail, ntt_pair};
+                                   reduce, plane_sum, equal, ntt_cluster, uniform_pairs, ntt_decrypt, tc_tail, ntt_pair};
     }
 
     const KernelTable* HMPC_CAT(kernel_table_, HMPC_L)()

@@ -29,6 +29,8 @@
 #include <cstdint>
 
 #include "chacha.cuh"
+#include "cast.cuh"
+#include "elementwise.cuh"
 #include "limbs.cuh"
 #include "ntt.cuh"
 
@@ -175,11 +177,13 @@ namespace hmpc_gb300
     }
 
     // One pass over the tiles of block `block` of the pass's grid.  exchange
-    // holds [2][L][blockDim.x] words.  Wait: whether the input may still be
-    // being written by the kernel before this one in the stream.
-    template<int L, int Kind, int NW, bool Inverse, bool Wait>
+    // holds [2][L][blockDim.x] words.  load and store take the polynomial (within
+    // its part), the index of the lower element of the thread's pair, the
+    // distance to the upper one, and the pair.  Wait: whether the input may
+    // still be being written by the kernel before this one in the stream.
+    template<int L, bool Inverse, bool Wait, class Load, class Store>
     __device__ __forceinline__ void ntt_pair_process(const PairPassParams& p, const Modulus<L>& m, uint64_t block,
-                                                     uint32_t* exchange)
+                                                     uint32_t* exchange, Load&& load, Store&& store)
     {
         const uint32_t t = threadIdx.x;
         const uint32_t w = p.w, c = p.c;
@@ -200,12 +204,10 @@ namespace hmpc_gb300
                 ++part;
             }
         }
-        uint32_t* const out_part = p.out[part];
         const uint32_t in_poly = static_cast<uint32_t>(tile) & ((1u << tile_bits) - 1u);
         const uint32_t mid_bits = p.row_shift - c;
         const uint32_t high = in_poly >> mid_bits;  // index bits above the rows
         const uint32_t base = (high << (p.row_shift + w)) | ((in_poly & ((1u << mid_bits) - 1u)) << c) | col;
-        const uint64_t poly_base = poly << p.log_n;
         // Stage j of the pass pairs row bit w-1-j (forward) or j (inverse).  The
         // thread bits above that one stand for the row bits above it, one to
         // one, so both the twiddle and the rows follow from r by shifts.
@@ -223,34 +225,14 @@ namespace hmpc_gb300
             const uint32_t row = Inverse ? r << 1 : r;
             const uint32_t idx = base | (row << p.row_shift);
             const uint32_t step = 1u << (p.row_shift + (Inverse ? 0u : w - 1));
-            if constexpr (Kind != producer_tensor)
+            if (active)
             {
-                if (active)
-                {
-                    if constexpr (Kind == producer_parts)
-                    {
-                        produce_part_pair<L>(p, m, part, poly, idx, step, lo, hi);
-                    }
-                    else
-                    {
-                        produce_pair<L, Kind, NW>(p, m, poly, idx, lo, hi);
-                    }
-                }
-                else
-                {
-                    set_zero<L>(lo);
-                    set_zero<L>(hi);
-                }
+                load(part, poly, idx, step, lo, hi);
             }
             else
             {
-                const uint32_t* in = (p.src ? p.src : out_part) + poly_base + idx;
-#pragma unroll
-                for (int j = 0; j < L; ++j)
-                {
-                    lo[j] = active ? in[static_cast<uint64_t>(j) * p.elements] : 0u;
-                    hi[j] = active ? in[static_cast<uint64_t>(j) * p.elements + step] : 0u;
-                }
+                set_zero<L>(lo);
+                set_zero<L>(hi);
             }
         }
         uint32_t* buffer = exchange;
@@ -337,22 +319,123 @@ namespace hmpc_gb300
         {
             const uint32_t row = Inverse ? r : r << 1;
             const uint32_t step = 1u << (p.row_shift + (Inverse ? w - 1 : 0u));
-            uint32_t* out = out_part + poly_base + (base | (row << p.row_shift));
-#pragma unroll
-            for (int j = 0; j < L; ++j)
-            {
-                out[static_cast<uint64_t>(j) * p.elements] = lo[j];
-                out[static_cast<uint64_t>(j) * p.elements + step] = hi[j];
-            }
+            store(part, poly, base | (row << p.row_shift), step, lo, hi);
         }
     }
 
+    // the pass's own input (tensor or sampler) and output
+    template<int L, int Kind, int NW, bool Inverse, bool Wait>
+    __device__ __forceinline__ void ntt_pair_pass(const PairPassParams& p, const Modulus<L>& m, uint64_t block,
+                                                  uint32_t* exchange)
+    {
+        ntt_pair_process<L, Inverse, Wait>(
+            p, m, block, exchange,
+            [&](uint32_t part, uint64_t poly, uint32_t idx, uint32_t step, uint32_t (&lo)[L], uint32_t (&hi)[L]) {
+                if constexpr (Kind == producer_parts)
+                {
+                    produce_part_pair<L>(p, m, part, poly, idx, step, lo, hi);
+                }
+                else if constexpr (Kind != producer_tensor)
+                {
+                    produce_pair<L, Kind, NW>(p, m, poly, idx, lo, hi);
+                }
+                else
+                {
+                    const uint32_t* in = (p.src ? p.src : p.out[part]) + (poly << p.log_n) + idx;
+                    load1<L>(lo, in, p.elements, 0);
+                    load1<L>(hi, in + step, p.elements, 0);
+                }
+            },
+            [&](uint32_t part, uint64_t poly, uint32_t idx, uint32_t step, const uint32_t (&lo)[L],
+                const uint32_t (&hi)[L]) {
+                uint32_t* out = p.out[part] + (poly << p.log_n) + idx;
+                store1<L>(out, p.elements, 0, lo);
+                store1<L>(out + step, p.elements, 0, hi);
+            });
+    }
+
+    // 64 registers at most (two blocks of 512 threads): at 8 limbs the inverse pass
+    // would take 72 and leave a second wave to batches that just fill the SMs (12
+    // of 2^13: 36.7 -> 25.0 us).  The parts' first pass, whose loads and keystream
+    // want more, stays without: 3 encryptions of 2^13 20.8 us, 23.9 with the limit.
     template<int L, int Kind, int NW, bool Inverse>
-    __global__ void __launch_bounds__(pair_max_threads, 2) ntt_pair_kernel(const PairPassParams p, const Modulus<L> m)
+    __global__ void __launch_bounds__(pair_max_threads, Kind == producer_parts ? 1 : 2)
+        ntt_pair_kernel(const PairPassParams p, const Modulus<L> m)
     {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         extern __shared__ uint32_t exchange[];
-        ntt_pair_process<L, Kind, NW, Inverse, true>(p, m, blockIdx.x, exchange);
+        ntt_pair_pass<L, Kind, NW, Inverse, true>(p, m, blockIdx.x, exchange);
+    }
+
+    // Decryption's inverse transform: the first pass forms its input c0 - s * c1
+    // (s broadcast over the batch; hmpc/expr/crypto/lhe/dec.hpp:29) as it loads,
+    // and the last pass lifts its result to the plaintext modulus (1 or 2 limbs)
+    // as it stores.
+    struct DecryptParams
+    {
+        const uint32_t* s;   // [L][N]
+        const uint32_t* c0;
+        const uint32_t* c1;
+        uint32_t* out;       // residues mod p, limb planes of `elements`
+        CastParams cast;
+        uint32_t p[2], pninv;
+    };
+
+    // LP: limbs of p in the last pass, 0 in the passes before it
+    template<int L, bool First, int LP>
+    __global__ void __launch_bounds__(pair_max_threads, 2) ntt_decrypt_kernel(const PairPassParams p,
+                                                                              const DecryptParams d,
+                                                                              const Modulus<L> m)
+    {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        extern __shared__ uint32_t exchange[];
+        ntt_pair_process<L, true, true>(
+            p, m, blockIdx.x, exchange,
+            [&](uint32_t, uint64_t poly, uint32_t idx, uint32_t step, uint32_t (&lo)[L], uint32_t (&hi)[L]) {
+                const uint64_t at = (poly << p.log_n) + idx;
+                if constexpr (First)
+                {
+                    auto combine = [&](uint32_t (&x)[L], uint32_t offset) {
+                        uint32_t t[L];
+                        load1<L>(x, d.s, 1ull << p.log_n, idx + offset);
+                        load1<L>(t, d.c1, p.elements, at + offset);
+                        mont_mul<L>(t, t, x, m);
+                        load1<L>(x, d.c0, p.elements, at + offset);
+                        mod_sub<L>(x, x, t, m);
+                    };
+                    combine(lo, 0);
+                    combine(hi, step);
+                }
+                else
+                {
+                    load1<L>(lo, p.out[0], p.elements, at);
+                    load1<L>(hi, p.out[0], p.elements, at + step);
+                }
+            },
+            [&](uint32_t, uint64_t poly, uint32_t idx, uint32_t step, const uint32_t (&lo)[L],
+                const uint32_t (&hi)[L]) {
+                const uint64_t at = (poly << p.log_n) + idx;
+                if constexpr (LP > 0)
+                {
+                    Modulus<LP> to;
+#pragma unroll
+                    for (int j = 0; j < LP; ++j)
+                    {
+                        to.q[j] = d.p[j];
+                    }
+                    to.ninv = d.pninv;
+                    uint32_t y[LP];
+                    cast_value<LP, L>(y, lo, d.cast, to);
+                    store1<LP>(d.out, p.elements, at, y);
+                    cast_value<LP, L>(y, hi, d.cast, to);
+                    store1<LP>(d.out, p.elements, at + step, y);
+                }
+                else
+                {
+                    store1<L>(p.out[0], p.elements, at, lo);
+                    store1<L>(p.out[0], p.elements, at + step, hi);
+                }
+            });
     }
 
     // ----------------------------------------------------------------------
@@ -436,7 +519,7 @@ namespace hmpc_gb300
                 return;
             }
             const PairPassParams& p = bp.params[bp.item_param[item]];
-            ntt_pair_process<L, producer_tensor, 1, Inverse, false>(p, m, bp.item_tile[item], exchange);
+            ntt_pair_pass<L, producer_tensor, 1, Inverse, false>(p, m, bp.item_tile[item], exchange);
             __syncthreads();
             if (threadIdx.x == 0)
             {
