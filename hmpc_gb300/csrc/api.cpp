@@ -82,7 +82,7 @@ namespace hmpc_gb300::detail
     }
 
     int run_transform(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, bool inverse, int kind,
-                      uint32_t vx2, uint32_t security, const uint32_t* src, uint32_t* out, const uint32_t* poly_rng,
+                      uint32_t vx2, uint32_t security, const uint32_t* src, uint32_t* out, const PolyRequest* requests,
                       uint32_t rng_slot, bool cuda_cores_only)
     {
         if (int rc = enter(ctx))
@@ -147,7 +147,7 @@ namespace hmpc_gb300::detail
         if (choice.radix_bits == 0)
         {
             // tensor-core engine; calls it does not cover run the default CUDA-core tiles
-            if (!cuda_cores_only && tc_applicable(mod, log_n, kind, poly_rng) &&
+            if (!cuda_cores_only && tc_applicable(mod, log_n, kind, requests) &&
                 (kind != producer_uniform || !inverse))
             {
                 if (kind != producer_uniform)
@@ -177,7 +177,7 @@ namespace hmpc_gb300::detail
         {
             // one thread-block cluster per polynomial; calls it does not cover
             // run the default CUDA-core tiles
-            if (kind == producer_tensor && !poly_rng && log_n >= 10 && log_n <= 14)
+            if (kind == producer_tensor && !requests && log_n >= 10 && log_n <= 14)
             {
                 ClusterNttParams cp{};
                 cp.in = src;
@@ -217,7 +217,7 @@ namespace hmpc_gb300::detail
             p.rng = ctx->rng();
             p.vx2 = vx2;
             p.top_mask = top_mask;
-            p.poly_rng = poly_rng;
+            p.requests = requests;
             p.rng_slot = rng_slot;
             cudaError_t e = mod->kt->ntt_pair(p, i == 0 ? kind : producer_tensor, nw, inverse, mod->h, plan[i].grid,
                                               plan[i].block, plan[i].smem, ctx->stream);
@@ -227,7 +227,7 @@ namespace hmpc_gb300::detail
             }
             ++ctx->launches;
         }
-        if (kind != producer_tensor && !poly_rng)
+        if (kind != producer_tensor && !requests)
         {
             nonce_add(ctx->nonce, n * batch);
         }
@@ -404,10 +404,10 @@ namespace hmpc_gb300::detail
 
     // Forward transforms of `count` parts of `batch` polynomials as one run of
     // passes: part i is drawn as kinds[i] with nonce ctx->nonce + slots[i] * n *
-    // batch (or from poly_rng's descriptors with that slot) and goes to out[i].
+    // batch (or from the requests' with that slot) and goes to out[i].
     int run_parts(hmpc_context* ctx, hmpc_modulus* q, const hmpc_modulus* p, uint64_t n, uint64_t batch, int count,
                   const uint32_t* kinds, const uint32_t* slots, uint32_t* const* out, const uint32_t* msg,
-                  const uint32_t* poly_rng)
+                  const PolyRequest* requests)
     {
         Tables* t = nullptr;
         if (int rc = q->prepare(n, &t))
@@ -424,7 +424,7 @@ namespace hmpc_gb300::detail
             pp.twiddles = t->forward;
             pp.small_table = q->small_table;
             pp.rng = ctx->rng();
-            pp.poly_rng = poly_rng;
+            pp.requests = requests;
             pp.dependent = dependent ? 1u : 0u;
             for (int j = 0; j < count; ++j)
             {
@@ -453,9 +453,44 @@ namespace hmpc_gb300::detail
         return HMPC_OK;
     }
 
+    int run_requests(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t polys, const PolyRequest* requests,
+                     bool& done)
+    {
+        const hmpc_modulus::TileChoice choice = mod->choice(n, false, polys);
+        done = choice.radix_bits >= 2;
+        if (!done)
+        {
+            return HMPC_OK;
+        }
+        Tables* t = nullptr;
+        if (int rc = mod->prepare(n, &t))
+        {
+            return rc;
+        }
+        const std::vector<PairPlan> plan =
+            plan_pairs(mod->c.limbs, __builtin_ctzll(n), polys, false, choice.local_bits, choice.col_bits);
+        const bool dependent = !capturing(ctx);
+        for (size_t i = 0; i < plan.size(); ++i)
+        {
+            PairPassParams p = plan[i].params;
+            p.dependent = dependent ? 1u : 0u;
+            p.twiddles = t->forward;
+            p.elements = n * polys;
+            p.requests = requests;
+            const cudaError_t e = mod->kt->ntt_request(p, i == 0, mod->h, plan[i].grid, plan[i].block, plan[i].smem,
+                                                       ctx->stream);
+            if (e != cudaSuccess)
+            {
+                return cuda_fail(e, "launching NTT pass");
+            }
+            ++ctx->launches;
+        }
+        return HMPC_OK;
+    }
+
     int encrypt_cuda_cores(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n, uint64_t batch,
                            const uint32_t* key_a, const uint32_t* key_b, const uint32_t* coefficients, uint32_t* c0,
-                           uint32_t* c1, uint32_t* workspace, const uint32_t* poly_rng, bool cuda_cores_only)
+                           uint32_t* c1, uint32_t* workspace, const PolyRequest* requests, bool cuda_cores_only)
     {
         const uint64_t elements = n * batch;
         const uint64_t poly_words = elements * static_cast<uint64_t>(q->c.limbs);
@@ -471,28 +506,29 @@ namespace hmpc_gb300::detail
             const uint32_t kinds[3] = {part_ternary, part_scaled_message, part_scaled};
             const uint32_t slots[3] = {0, 1, 2};
             uint32_t* const outs[3] = {u, v, msg};
-            if (int rc = run_parts(ctx, q, p, n, batch, 3, kinds, slots, outs, coefficients, poly_rng))
+            if (int rc = run_parts(ctx, q, p, n, batch, 3, kinds, slots, outs, coefficients, requests))
             {
                 return rc;
             }
-            cudaError_t e = q->kt->lhe_combine_pair(c0, c1, key_a, key_b, n, u, v, msg, elements, elements,
+            cudaError_t e = q->kt->lhe_combine_pair(c0, c1, c0 ? nullptr : requests, key_a, key_b, n, u, v, msg,
+                                                    elements, elements,
                                                     !capturing(ctx), q->h, ctx->stream);
             if (e != cudaSuccess)
             {
                 return cuda_fail(e, "launching combine");
             }
             ++ctx->launches;
-            if (!poly_rng)
+            if (!requests)
             {
                 nonce_add(ctx->nonce, 3 * elements);
             }
             return HMPC_OK;
         }
         // the reference's plan: NTT(u), NTT(v), NTT_q(msg), c0, NTT(w), c1
-        int rc = run_transform(ctx, q, n, batch, false, producer_cbd, 1, 0, nullptr, u, poly_rng, 0, cuda_cores_only);
+        int rc = run_transform(ctx, q, n, batch, false, producer_cbd, 1, 0, nullptr, u, requests, 0, cuda_cores_only);
         if (!rc)
         {
-            rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v, poly_rng, 1, cuda_cores_only);
+            rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v, requests, 1, cuda_cores_only);
         }
         if (rc)
         {
@@ -516,7 +552,7 @@ namespace hmpc_gb300::detail
         }
         ++ctx->launches;
         // w reuses v's buffer
-        if ((rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v, poly_rng, 2,
+        if ((rc = run_transform(ctx, q, n, batch, false, producer_cbd, 20, 0, nullptr, v, requests, 2,
                                 cuda_cores_only)))
         {
             return rc;

@@ -64,12 +64,13 @@ namespace hmpc_gb300
         cudaError_t (*ntt_batched)(const BatchedParams& bp, bool inverse, const HostModulus& m, unsigned grid,
                                    unsigned block, size_t smem, cudaStream_t stream);
         int (*ntt_batched_blocks_per_sm)(bool inverse, unsigned block, size_t smem);
-        // u, x, w: limb planes of `stride` words; dependent: launch with
+        // into c0 and c1 or, with requests, into each polynomial's request's
+        // outputs; u, x, w: limb planes of `stride` words; dependent: launch with
         // programmatic dependence on the kernel before it in the stream
-        cudaError_t (*lhe_combine_pair)(uint32_t* c0, uint32_t* c1, const uint32_t* ka, const uint32_t* kb,
-                                        uint64_t n, const uint32_t* u, const uint32_t* x, const uint32_t* w,
-                                        uint64_t stride, uint64_t elements, bool dependent, const HostModulus& m,
-                                        cudaStream_t stream);
+        cudaError_t (*lhe_combine_pair)(uint32_t* c0, uint32_t* c1, const PolyRequest* requests, const uint32_t* ka,
+                                        const uint32_t* kb, uint64_t n, const uint32_t* u, const uint32_t* x,
+                                        const uint32_t* w, uint64_t stride, uint64_t elements, bool dependent,
+                                        const HostModulus& m, cudaStream_t stream);
         cudaError_t (*lhe_key)(uint32_t* a, uint32_t* b, const uint32_t* s, const uint32_t* x, uint64_t elements,
                                const RngKey& rng, int words, uint32_t top_mask, bool dependent, const HostModulus& m,
                                cudaStream_t stream);
@@ -94,6 +95,9 @@ namespace hmpc_gb300
         // (for the tensor-core engine, whose first group reads memory)
         cudaError_t (*uniform_pairs)(uint32_t* out, uint32_t log_n, uint64_t elements, const RngKey& rng,
                                      int words, uint32_t top_mask, const HostModulus& m, cudaStream_t stream);
+        // one forward pass over p.requests' own buffers
+        cudaError_t (*ntt_request)(const PairPassParams& p, bool first, const HostModulus& m, unsigned grid,
+                                   unsigned block, size_t smem, cudaStream_t stream);
         // one pass of a decryption's inverse transform; p_limbs: 1 or 2 in the
         // last pass, else 0
         cudaError_t (*ntt_decrypt)(const PairPassParams& p, const DecryptParams& d, bool first, int p_limbs,

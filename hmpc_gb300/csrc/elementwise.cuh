@@ -10,6 +10,7 @@
 
 #include "chacha.cuh"
 #include "limbs.cuh"
+#include "ntt.cuh"
 
 namespace hmpc_gb300
 {
@@ -174,9 +175,11 @@ namespace hmpc_gb300
     // (linearity of the NTT).  u, x and w have `stride` words per limb plane;
     // u is read once for both products.  One element per thread (about 50
     // registers at L = 8): enough resident warps to cover the loads' latency
-    // with the products' arithmetic.  n is a power of two.
-    template<int L>
-    __global__ void __launch_bounds__(256) lhe_combine_pair_kernel(uint32_t* c0, uint32_t* c1, const uint32_t* ka,
+    // with the products' arithmetic.  n is a power of two.  Requests: c0 and c1
+    // are the outputs of each polynomial's request.
+    template<int L, bool Requests>
+    __global__ void __launch_bounds__(256) lhe_combine_pair_kernel(uint32_t* c0, uint32_t* c1,
+                                                                   const PolyRequest* requests, const uint32_t* ka,
                                                                    const uint32_t* kb, uint64_t n,
                                                                    const uint32_t* u_planes,
                                                                    const uint32_t* x_planes,
@@ -188,18 +191,28 @@ namespace hmpc_gb300
         for (uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < elements;
              e += static_cast<uint64_t>(gridDim.x) * blockDim.x)
         {
+            uint32_t* out0 = c0 + e;
+            uint32_t* out1 = c1 + e;
+            uint64_t out_stride = elements;
+            if constexpr (Requests)
+            {
+                const PolyRequest& d = requests[e / n];
+                out0 = d.out[0] + (e & mask);
+                out1 = d.out[1] + (e & mask);
+                out_stride = d.stride;
+            }
             uint32_t u[L], k[L], x[L];
             load1<L>(u, u_planes, stride, e);
             load1<L>(k, ka, n, e & mask);
             load1<L>(x, x_planes, stride, e);
             mont_mul<L>(k, k, u, m);
             mod_add<L>(x, x, k, m);
-            store1<L>(c0, elements, e, x);
+            store1<L>(out0, out_stride, 0, x);
             load1<L>(k, kb, n, e & mask);
             load1<L>(x, w_planes, stride, e);
             mont_mul<L>(k, k, u, m);
             mod_add<L>(x, x, k, m);
-            store1<L>(c1, elements, e, x);
+            store1<L>(out1, out_stride, 0, x);
         }
     }
 

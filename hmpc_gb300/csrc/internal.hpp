@@ -276,23 +276,32 @@ namespace hmpc_gb300::detail
     // cuda_cores_only: ignore a tensor-core plan (callers that must not allocate)
     int run_transform(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, bool inverse, int kind,
                       uint32_t vx2, uint32_t security, const uint32_t* src, uint32_t* out,
-                      const uint32_t* poly_rng = nullptr, uint32_t rng_slot = 0, bool cuda_cores_only = false);
+                      const PolyRequest* requests = nullptr, uint32_t rng_slot = 0, bool cuda_cores_only = false);
     int run_plain(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, bool inverse, int kind,
                   uint32_t vx2, uint32_t security, const uint32_t* src, uint32_t* out);
     CastParams make_cast(const hmpc_modulus* dst, const hmpc_modulus* src);
     bool capturing(const hmpc_context* ctx);
+    // whether an encryption's (or key pair's) transforms run as parts of one set
+    // of passes
+    bool parts_applicable(const hmpc_modulus* q, const hmpc_modulus* p);
     // BGV encryption on the CUDA cores from coefficient-form plaintexts, 3 *
-    // batch * n * L_q words of workspace; poly_rng: per-polynomial RNG
-    // descriptors of independent requests (the context's nonce stays)
+    // batch * n * L_q words of workspace.  requests (device memory, one per
+    // polynomial): independent requests with nonces of their own (the context's
+    // stays); where parts_applicable, coefficients, c0 and c1 may be nullptr, and
+    // the requests' own buffers are read and written.
     int encrypt_cuda_cores(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n, uint64_t batch,
                            const uint32_t* key_a, const uint32_t* key_b, const uint32_t* coefficients, uint32_t* c0,
-                           uint32_t* c1, uint32_t* workspace, const uint32_t* poly_rng, bool cuda_cores_only);
+                           uint32_t* c1, uint32_t* workspace, const PolyRequest* requests, bool cuda_cores_only);
+    // forward transforms of `polys` polynomials of degree n between the requests'
+    // own buffers, if the shape's plan is a CUDA-core one (else done = false)
+    int run_requests(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t polys, const PolyRequest* requests,
+                     bool& done);
     // tensor-core engine: whether the modulus qualifies (2 to 8 limbs, q
     // below 0.996 * 2^(32L), top limb at least 32) and whether a call does
     // (forward from a tensor or CBD(V) samples, or inverse; at least 16
     // coefficients; no per-polynomial RNG)
     bool tc_supported(const hmpc_modulus* mod);
-    bool tc_applicable(const hmpc_modulus* mod, int log_n, int kind, const uint32_t* poly_rng);
+    bool tc_applicable(const hmpc_modulus* mod, int log_n, int kind, const PolyRequest* requests);
     // splits: output split of the group whose rows are contiguous (1 or 2)
     int run_tc_transform(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, bool inverse, int kind,
                          uint32_t vx2, const uint32_t* src, uint32_t* out, int splits,

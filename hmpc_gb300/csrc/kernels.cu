@@ -372,16 +372,17 @@ namespace hmpc_gb300
             return e == cudaSuccess ? blocks : 0;
         }
 
-        cudaError_t lhe_combine_pair(uint32_t* c0, uint32_t* c1, const uint32_t* ka, const uint32_t* kb, uint64_t n,
-                                     const uint32_t* u, const uint32_t* x, const uint32_t* w, uint64_t stride,
+        cudaError_t lhe_combine_pair(uint32_t* c0, uint32_t* c1, const PolyRequest* requests, const uint32_t* ka,
+                                     const uint32_t* kb, uint64_t n, const uint32_t* u, const uint32_t* x, const uint32_t* w, uint64_t stride,
                                      uint64_t elements, bool dependent, const HostModulus& h, cudaStream_t stream)
         {
             if (elements == 0)
             {
                 return cudaSuccess;
             }
-            return launch(lhe_combine_pair_kernel<L>, grid_for(elements, 256), 256, 0, dependent, stream, c0, c1, ka,
-                          kb, n, u, x, w, stride, elements, device_modulus(h));
+            return launch(requests ? lhe_combine_pair_kernel<L, true> : lhe_combine_pair_kernel<L, false>,
+                          grid_for(elements, 256), 256, 0, dependent, stream, c0, c1, requests, ka, kb, n, u, x, w,
+                          stride, elements, device_modulus(h));
         }
 
         cudaError_t lhe_key(uint32_t* a, uint32_t* b, const uint32_t* s, const uint32_t* x, uint64_t elements,
@@ -468,6 +469,13 @@ namespace hmpc_gb300
             return cudaGetLastError();
         }
 
+        cudaError_t ntt_request(const PairPassParams& p, bool first, const HostModulus& h, unsigned grid,
+                                unsigned block, size_t smem, cudaStream_t stream)
+        {
+            return launch(first ? ntt_request_kernel<L, true> : ntt_request_kernel<L, false>, grid, block, smem,
+                          p.dependent != 0, stream, p, device_modulus(h));
+        }
+
         cudaError_t ntt_decrypt(const PairPassParams& p, const DecryptParams& d, bool first, int p_limbs,
                                 const HostModulus& h, unsigned grid, unsigned block, size_t smem, cudaStream_t stream)
         {
@@ -519,7 +527,7 @@ namespace hmpc_gb300
         const KernelTable table = {fma, binary, lhe_combine, uniform, cbd, to_montgomery,
                                    from_montgomery, cast, plain_stage, ct_mul, dec_combine, ntt_batched,
                                    ntt_batched_blocks_per_sm, lhe_combine_pair, lhe_key, matvec, matvec_monomial,
-                                   reduce, plane_sum, equal, ntt_cluster, uniform_pairs, ntt_decrypt, tc_tail, ntt_pair};
+                                   reduce, plane_sum, equal, ntt_cluster, uniform_pairs, ntt_request, ntt_decrypt, tc_tail, ntt_pair};
     }
 
     const KernelTable* HMPC_CAT(kernel_table_, HMPC_L)()

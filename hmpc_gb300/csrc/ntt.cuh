@@ -20,27 +20,39 @@ namespace hmpc_gb300
         producer_parts = 3,    // the parts of an encryption or key pair (PairParts)
     };
 
+    // One polynomial of a batch of independent requests: its RNG (the request's
+    // nonce, the polynomial's index in the request and the request's polynomial
+    // count), and where its coefficients are in the request's own buffers, limb
+    // planes `stride` words apart.
+    struct PolyRequest
+    {
+        uint32_t nonce[3];
+        uint32_t index, count;
+        const uint32_t* in;
+        uint32_t* out[2];
+        uint64_t stride;
+    };
+
     // Generator key, nonce and counter of the stage-0 pair whose first element
-    // is coefficient idx_u of polynomial `poly`.  With per-polynomial RNG
-    // (batches of independent requests: p.poly_rng), polynomial i draws with
-    // nonce = desc[0..2] + slot * desc[4] * N and counter = desc[3] * N +
-    // coefficient, desc = poly_rng + 5 i -- exactly what the request would draw
-    // alone with its own nonce.
+    // is coefficient idx_u of polynomial `poly`.  With p.requests, polynomial i
+    // draws with nonce = requests[i].nonce + slot * count * N and counter = index
+    // * N + coefficient -- exactly what the request would draw alone with its own
+    // nonce.
     template<class Params>
     __device__ __forceinline__ uint32_t pair_generator(const Params& p, uint64_t poly, uint64_t idx_u, uint32_t slot,
                                                        RngKey& rng)
     {
         rng = p.rng;
-        if (p.poly_rng)
+        if (p.requests)
         {
-            const uint32_t* d = p.poly_rng + poly * 5;
-            const uint64_t add = static_cast<uint64_t>(slot) * d[4] << p.log_n;
-            uint64_t s = static_cast<uint64_t>(d[0]) + static_cast<uint32_t>(add);
+            const PolyRequest& d = p.requests[poly];
+            const uint64_t add = static_cast<uint64_t>(slot) * d.count << p.log_n;
+            uint64_t s = static_cast<uint64_t>(d.nonce[0]) + static_cast<uint32_t>(add);
             rng.nonce[0] = static_cast<uint32_t>(s);
-            s = static_cast<uint64_t>(d[1]) + static_cast<uint32_t>(add >> 32) + (s >> 32);
+            s = static_cast<uint64_t>(d.nonce[1]) + static_cast<uint32_t>(add >> 32) + (s >> 32);
             rng.nonce[1] = static_cast<uint32_t>(s);
-            rng.nonce[2] = d[2] + static_cast<uint32_t>(s >> 32);
-            return static_cast<uint32_t>((static_cast<uint64_t>(d[3]) << p.log_n) + idx_u);
+            rng.nonce[2] = d.nonce[2] + static_cast<uint32_t>(s >> 32);
+            return static_cast<uint32_t>((static_cast<uint64_t>(d.index) << p.log_n) + idx_u);
         }
         return static_cast<uint32_t>(poly * (1ull << p.log_n) + idx_u);
     }

@@ -54,7 +54,8 @@ namespace hmpc_gb300
     {
         uint32_t kind[pair_max_parts];
         uint32_t nonce[pair_max_parts][3];
-        const uint32_t* msg;           // msg_limbs planes of `elements` words, Montgomery form
+        const uint32_t* msg;           // msg_limbs planes of `elements` words, Montgomery form (nullptr: the
+                                       // requests' inputs)
         uint32_t msg_limbs;
         uint32_t pq[2], phalf[2], pninv;
         uint32_t r2[9];                // R^2 mod Q
@@ -75,7 +76,7 @@ namespace hmpc_gb300
         RngKey rng;
         uint32_t vx2;                  // 2V for the CBD producer
         uint32_t top_mask;             // uniform producer: mask of the top word
-        const uint32_t* poly_rng;      // per-polynomial RNG, see pair_generator
+        const PolyRequest* requests;   // one per polynomial of a part (nullptr: none)
         uint32_t rng_slot;
         uint32_t dependent;            // host side: programmatic dependence on the kernel before
         PairParts parts;               // parts producer
@@ -139,18 +140,20 @@ namespace hmpc_gb300
         if (kind == part_scaled_message)
         {
             // issued before the keystream is computed: their latency hides behind it
-            const uint32_t* at = p.parts.msg + (poly << p.log_n) + idx;
+            const uint32_t* at = p.parts.msg ? p.parts.msg + (poly << p.log_n) : p.requests[poly].in;
+            const uint64_t plane = p.parts.msg ? p.elements : p.requests[poly].stride;
+            at += idx;
             msg[0][0] = at[0];
             msg[1][0] = at[step];
             if (p.parts.msg_limbs > 1)
             {
-                msg[0][1] = at[p.elements];
-                msg[1][1] = at[p.elements + step];
+                msg[0][1] = at[plane];
+                msg[1][1] = at[plane + step];
             }
         }
         RngKey rng;
         const uint32_t counter = pair_generator(p, poly, idx, part, rng);
-        if (!p.poly_rng)
+        if (!p.requests)
         {
             rng.nonce[0] = p.parts.nonce[part][0];
             rng.nonce[1] = p.parts.nonce[part][1];
@@ -365,6 +368,30 @@ namespace hmpc_gb300
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         extern __shared__ uint32_t exchange[];
         ntt_pair_pass<L, Kind, NW, Inverse, true>(p, m, blockIdx.x, exchange);
+    }
+
+    // Forward passes over the requests' own buffers: the first reads their
+    // inputs, every one writes their outputs.
+    template<int L, bool First>
+    __global__ void __launch_bounds__(pair_max_threads, 2) ntt_request_kernel(const PairPassParams p,
+                                                                              const Modulus<L> m)
+    {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        extern __shared__ uint32_t exchange[];
+        ntt_pair_process<L, false, true>(
+            p, m, blockIdx.x, exchange,
+            [&](uint32_t, uint64_t poly, uint32_t idx, uint32_t step, uint32_t (&lo)[L], uint32_t (&hi)[L]) {
+                const PolyRequest& d = p.requests[poly];
+                const uint32_t* in = (First ? d.in : d.out[0]) + idx;
+                load1<L>(lo, in, d.stride, 0);
+                load1<L>(hi, in + step, d.stride, 0);
+            },
+            [&](uint32_t, uint64_t poly, uint32_t idx, uint32_t step, const uint32_t (&lo)[L],
+                const uint32_t (&hi)[L]) {
+                const PolyRequest& d = p.requests[poly];
+                store1<L>(d.out[0] + idx, d.stride, 0, lo);
+                store1<L>(d.out[0] + idx + step, d.stride, 0, hi);
+            });
     }
 
     // Decryption's inverse transform: the first pass forms its input c0 - s * c1

@@ -10,7 +10,7 @@
 // and twiddle tables stay resident.  Every request's result is the result it
 // would have alone: transforms and products have no state, and an encryption
 // draws its randomness from its own nonce with coefficient indices local to
-// the request (per-polynomial RNG descriptors), whatever batch it lands in.
+// the request (per-polynomial descriptors), whatever batch it lands in.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -135,12 +135,12 @@ struct hmpc_server
     uint32_t max_batch = 16;
     std::vector<std::unique_ptr<hmpc_context>> lanes;
     std::vector<cudaEvent_t> lane_done;
-    std::vector<uint32_t*> lane_desc;        // pinned RNG descriptors per lane
+    std::vector<PolyRequest*> lane_desc;     // pinned descriptors per lane
     std::vector<Dispatch> lane_work;
     std::vector<bool> lane_busy;
     uint32_t desc_capacity = 0;              // polynomials per lane descriptor buffer
     uint32_t batch_window_us = 0;            // hold a group that is not full for compatible arrivals
-    uint32_t* d_desc = nullptr;              // device descriptors, one region per lane
+    PolyRequest* d_desc = nullptr;           // device descriptors, one region per lane
     uint8_t* pool_base = nullptr;
     Pool pool;
     std::vector<ResidentKey> keys;
@@ -225,6 +225,34 @@ struct hmpc_server
                                  static_cast<size_t>(limbs), cudaMemcpyDeviceToDevice, s);
     }
 
+    // the descriptors of a dispatch's polynomials, on their way to the lane's
+    // region of device memory
+    int describe(Dispatch& d, uint64_t n, uint64_t polys, const PolyRequest** out)
+    {
+        PolyRequest* host_desc = lane_desc[static_cast<size_t>(d.lane)];
+        PolyRequest* dev_desc = d_desc + static_cast<uint64_t>(d.lane) * desc_capacity;
+        uint64_t poly = 0;
+        for (auto* x : d.reqs)
+        {
+            for (uint64_t j = 0; j < x->r.count; ++j, ++poly)
+            {
+                PolyRequest& desc = host_desc[poly];
+                std::copy(x->r.nonce, x->r.nonce + 3, desc.nonce);
+                desc.index = static_cast<uint32_t>(j);
+                desc.count = static_cast<uint32_t>(x->r.count);
+                desc.in = x->r.in0 + j * n;
+                desc.out[0] = x->r.out0 + j * n;
+                desc.out[1] = x->r.out1 ? x->r.out1 + j * n : nullptr;
+                desc.stride = n * x->r.count;
+            }
+        }
+        HMPC_CUDA(cudaMemcpyAsync(dev_desc, host_desc, polys * sizeof(PolyRequest), cudaMemcpyHostToDevice,
+                                  lanes[static_cast<size_t>(d.lane)]->stream),
+                  "uploading request descriptors");
+        *out = dev_desc;
+        return HMPC_OK;
+    }
+
     int issue(Dispatch& d)
     {
         hmpc_context* lane = lanes[static_cast<size_t>(d.lane)].get();
@@ -267,6 +295,18 @@ struct hmpc_server
             if (single)
             {
                 return run_transform(lane, q, r0.n, r0.count, false, producer_tensor, 0, 0, r0.in0, r0.out0);
+            }
+            // between the requests' own buffers, unless their plan is an engine
+            // that works on one buffer
+            const PolyRequest* dev_desc = nullptr;
+            if (int rc = describe(d, r0.n, polys, &dev_desc))
+            {
+                return rc;
+            }
+            bool done = false;
+            if (int rc = run_requests(lane, q, r0.n, polys, dev_desc, done); rc || done)
+            {
+                return rc;
             }
             const uint64_t total = r0.n * polys;
             uint64_t at = 0;
@@ -315,23 +355,16 @@ struct hmpc_server
         uint32_t* pt = scratch + 3 * qw;
         uint32_t* c0 = pt + total * static_cast<uint64_t>(lp);
         uint32_t* c1 = c0 + qw;
-        uint32_t* host_desc = lane_desc[static_cast<size_t>(d.lane)];
-        uint32_t* dev_desc = d_desc + static_cast<uint64_t>(d.lane) * desc_capacity * 5;
-        uint64_t poly = 0;
-        for (auto* x : d.reqs)
+        const PolyRequest* dev_desc = nullptr;
+        if (int rc = describe(d, n, polys, &dev_desc))
         {
-            for (uint64_t j = 0; j < x->r.count; ++j, ++poly)
-            {
-                uint32_t* desc = host_desc + poly * 5;
-                desc[0] = x->r.nonce[0];
-                desc[1] = x->r.nonce[1];
-                desc[2] = x->r.nonce[2];
-                desc[3] = static_cast<uint32_t>(j);
-                desc[4] = static_cast<uint32_t>(x->r.count);
-            }
+            return rc;
         }
-        HMPC_CUDA(cudaMemcpyAsync(dev_desc, host_desc, polys * 5 * sizeof(uint32_t), cudaMemcpyHostToDevice, s),
-                  "uploading RNG descriptors");
+        if (parts_applicable(k.q, k.p))
+        {
+            return encrypt_cuda_cores(lane, k.q, k.p, n, polys, k.a, k.b, nullptr, nullptr, nullptr, scratch, dev_desc,
+                                      false);
+        }
         const uint32_t* plaintext = r0.in0;
         if (!single)
         {
@@ -551,15 +584,15 @@ int hmpc_server_create(hmpc_context* ctx, const hmpc_server_config* config, hmpc
         HMPC_CUDA(cudaStreamCreateWithFlags(&lane->stream, cudaStreamNonBlocking), "creating a lane stream");
         cudaEvent_t ev;
         HMPC_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "creating a lane event");
-        uint32_t* desc = nullptr;
-        HMPC_CUDA(cudaMallocHost(&desc, srv->desc_capacity * 5ull * sizeof(uint32_t)), "allocating descriptors");
+        PolyRequest* desc = nullptr;
+        HMPC_CUDA(cudaMallocHost(&desc, srv->desc_capacity * sizeof(PolyRequest)), "allocating descriptors");
         srv->lanes.push_back(std::move(lane));
         srv->lane_done.push_back(ev);
         srv->lane_desc.push_back(desc);
     }
     srv->lane_work.resize(config->lanes);
     srv->lane_busy.assign(config->lanes, false);
-    HMPC_CUDA(cudaMalloc(&srv->d_desc, srv->desc_capacity * 5ull * config->lanes * sizeof(uint32_t)),
+    HMPC_CUDA(cudaMalloc(&srv->d_desc, srv->desc_capacity * static_cast<uint64_t>(config->lanes) * sizeof(PolyRequest)),
               "allocating descriptors");
     if (config->memory_budget_bytes)
     {

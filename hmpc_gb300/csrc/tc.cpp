@@ -494,9 +494,9 @@ namespace hmpc_gb300::detail
         return !inverse && n >= 512 && mod->c.bits >= 32 * mod->c.limbs - 14;
     }
 
-    bool tc_applicable(const hmpc_modulus* mod, int log_n, int kind, const uint32_t* poly_rng)
+    bool tc_applicable(const hmpc_modulus* mod, int log_n, int kind, const PolyRequest* requests)
     {
-        return log_n >= 4 && !poly_rng && (kind == producer_tensor || kind == producer_cbd || kind == producer_uniform) &&
+        return log_n >= 4 && !requests && (kind == producer_tensor || kind == producer_cbd || kind == producer_uniform) &&
                tc_supported(mod);
     }
 
@@ -941,7 +941,7 @@ namespace hmpc_gb300::detail
         }
         if (!tt->tail)
         {
-            cudaError_t e = mod->kt->lhe_combine_pair(combine.c0, combine.c1, combine.key_a, combine.key_b, n, stacked,
+            cudaError_t e = mod->kt->lhe_combine_pair(combine.c0, combine.c1, nullptr, combine.key_a, combine.key_b, n, stacked,
                                                       stacked + elements, stacked + 2 * elements, total, elements,
                                                       !capturing(ctx), mod->h, ctx->stream);
             if (e != cudaSuccess)
