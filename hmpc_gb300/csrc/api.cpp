@@ -291,13 +291,21 @@ namespace hmpc_gb300::detail
 
     // the lift of INTT_q(c0 - s*c1) to p in the inverse transform's own passes
     int run_decrypt(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_t n, uint64_t batch, const uint32_t* s,
-                    const uint32_t* c0, const uint32_t* c1, uint32_t* x, uint32_t* out,
-                    const std::vector<PairPlan>& plan)
+                    const uint32_t* c0, const uint32_t* c1, uint32_t* x, uint32_t* out, bool ntt_form,
+                    const hmpc_modulus::TileChoice& choice, const std::vector<PairPlan>& plan)
     {
         Tables* t = nullptr;
+        Tables* pt = nullptr;
         if (int rc = q->prepare(n, &t))
         {
             return rc;
+        }
+        if (ntt_form)
+        {
+            if (int rc = p->prepare(n, &pt))
+            {
+                return rc;
+            }
         }
         DecryptParams d{};
         d.s = s;
@@ -307,6 +315,7 @@ namespace hmpc_gb300::detail
         d.cast = make_cast(p, q);
         std::copy(p->h.q, p->h.q + p->c.limbs, d.p);
         d.pninv = p->h.ninv;
+        d.p_twiddles = ntt_form ? pt->forward : nullptr;
         const bool dependent = !capturing(ctx);
         for (size_t i = 0; i < plan.size(); ++i)
         {
@@ -320,6 +329,28 @@ namespace hmpc_gb300::detail
             if (e != cudaSuccess)
             {
                 return cuda_fail(e, "launching decryption pass");
+            }
+            ++ctx->launches;
+        }
+        if (!ntt_form)
+        {
+            return HMPC_OK;
+        }
+        // the forward transform mod p from its second pass on, in the same tiles
+        const std::vector<PairPlan> forward =
+            plan_pairs(p->c.limbs, __builtin_ctzll(n), batch, false, choice.local_bits, choice.col_bits);
+        for (size_t i = 1; i < forward.size(); ++i)
+        {
+            PairPassParams pp = forward[i].params;
+            pp.out[0] = out;
+            pp.twiddles = pt->forward;
+            pp.elements = n * batch;
+            pp.dependent = dependent ? 1u : 0u;
+            const cudaError_t e = p->kt->ntt_pair(pp, producer_tensor, 1, false, p->h, forward[i].grid,
+                                                  forward[i].block, forward[i].smem, ctx->stream);
+            if (e != cudaSuccess)
+            {
+                return cuda_fail(e, "launching NTT pass");
             }
             ++ctx->launches;
         }
@@ -364,12 +395,7 @@ namespace hmpc_gb300::detail
             if (plan.size() > 1 || !(overlap(out, out_words, c0, q_words) || overlap(out, out_words, c1, q_words) ||
                                      overlap(out, out_words, s, s_words)))
             {
-                if (int rc = run_decrypt(ctx, q, p, n, batch, s, c0, c1, x, out, plan))
-                {
-                    return rc;
-                }
-                return plaintext_ntt ? run_transform(ctx, p, n, batch, false, producer_tensor, 0, 0, out, out)
-                                     : HMPC_OK;
+                return run_decrypt(ctx, q, p, n, batch, s, c0, c1, x, out, plaintext_ntt != 0, choice, plan);
             }
         }
         cudaError_t e = q->kt->dec_combine(x, s, n, c0, c1, c2, elements, q->h, ctx->stream);

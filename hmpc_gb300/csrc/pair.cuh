@@ -179,73 +179,41 @@ namespace hmpc_gb300
         int_to_mont<L>(v, y, p.parts.r2, m);
     }
 
-    // One pass over the tiles of block `block` of the pass's grid.  exchange
-    // holds [2][L][blockDim.x] words.  load and store take the polynomial (within
-    // its part), the index of the lower element of the thread's pair, the
-    // distance to the upper one, and the pair.  Wait: whether the input may
-    // still be being written by the kernel before this one in the stream.
-    template<int L, bool Inverse, bool Wait, class Load, class Store>
-    __device__ __forceinline__ void ntt_pair_process(const PairPassParams& p, const Modulus<L>& m, uint64_t block,
-                                                     uint32_t* exchange, Load&& load, Store&& store)
+    // A thread's place in a tile.  Stage j of the pass pairs row bit w-1-j
+    // (forward) or j (inverse).  The thread bits above that one stand for the
+    // row bits above it, one to one, so both the twiddle and the rows follow from
+    // r by shifts.
+    struct PairTile
+    {
+        uint32_t w, c;
+        uint32_t r;             // the row bits but the pair's
+        uint32_t twiddle_high;  // from the index bits above the rows
+        uint32_t* buffer;       // the exchange buffers, taking turns
+        uint32_t* other;
+
+        template<bool Inverse>
+        __device__ __forceinline__ uint32_t twiddle_index(uint32_t j) const
+        {
+            return Inverse ? (twiddle_high << (w - 1 - j)) + (r >> j) : (twiddle_high << j) + (r >> (w - 1 - j));
+        }
+    };
+
+    // The stages of a pass on the pair (lo, hi), tw the first stage's twiddle; by
+    // every thread of the block.  last: the inverse transform's last stage is the
+    // pass's last.
+    template<int L, bool Inverse>
+    __device__ __forceinline__ void pair_stages(uint32_t (&lo)[L], uint32_t (&hi)[L], uint32_t (&tw)[L],
+                                                PairTile& tile, const uint32_t* twiddles, bool last,
+                                                const Modulus<L>& m)
     {
         const uint32_t t = threadIdx.x;
-        const uint32_t w = p.w, c = p.c;
-        const uint32_t pair_bits = w + c - 1;
-        const uint64_t tile = block * (blockDim.x >> pair_bits) + (t >> pair_bits);
-        const bool active = tile < p.tiles;
-        const uint32_t col = t & ((1u << c) - 1u);
-        const uint32_t r = (t >> c) & ((1u << (w - 1)) - 1u);  // the row bits but the pair's
-        const uint32_t tile_bits = p.log_n - w - c;
-        uint64_t poly = tile >> tile_bits;
-        uint32_t part = 0;
-#pragma unroll
-        for (int i = 1; i < pair_max_parts; ++i)
-        {
-            if (poly >= p.part_polys)
-            {
-                poly -= p.part_polys;
-                ++part;
-            }
-        }
-        const uint32_t in_poly = static_cast<uint32_t>(tile) & ((1u << tile_bits) - 1u);
-        const uint32_t mid_bits = p.row_shift - c;
-        const uint32_t high = in_poly >> mid_bits;  // index bits above the rows
-        const uint32_t base = (high << (p.row_shift + w)) | ((in_poly & ((1u << mid_bits) - 1u)) << c) | col;
-        // Stage j of the pass pairs row bit w-1-j (forward) or j (inverse).  The
-        // thread bits above that one stand for the row bits above it, one to
-        // one, so both the twiddle and the rows follow from r by shifts.
-        const uint32_t twiddle_high = (1u << (p.log_n - p.row_shift - w)) + high;
-        auto twiddle_index = [&](uint32_t j) {
-            return Inverse ? (twiddle_high << (w - 1 - j)) + (r >> j) : (twiddle_high << j) + (r >> (w - 1 - j));
-        };
-        uint32_t lo[L], hi[L], tw[L];
-        load_twiddle<L>(tw, p.twiddles, twiddle_index(0));
-        if constexpr (Wait)
-        {
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-        }
-        {
-            const uint32_t row = Inverse ? r << 1 : r;
-            const uint32_t idx = base | (row << p.row_shift);
-            const uint32_t step = 1u << (p.row_shift + (Inverse ? 0u : w - 1));
-            if (active)
-            {
-                load(part, poly, idx, step, lo, hi);
-            }
-            else
-            {
-                set_zero<L>(lo);
-                set_zero<L>(hi);
-            }
-        }
-        uint32_t* buffer = exchange;
-        uint32_t* other = exchange + L * blockDim.x;
+        const uint32_t w = tile.w;
 #pragma unroll 1
         for (uint32_t j = 0; j < w; ++j)
         {
             if (j > 0)
             {
-                const uint32_t bit = c + (Inverse ? j - 1 : w - 1 - j);
+                const uint32_t bit = tile.c + (Inverse ? j - 1 : w - 1 - j);
                 const bool upper = (t >> bit) & 1u;
                 if (bit < 5)
                 {
@@ -262,25 +230,25 @@ namespace hmpc_gb300
 #pragma unroll
                     for (int k = 0; k < L; ++k)
                     {
-                        buffer[k * blockDim.x + t] = upper ? lo[k] : hi[k];
+                        tile.buffer[k * blockDim.x + t] = upper ? lo[k] : hi[k];
                     }
                     __syncthreads();
 #pragma unroll
                     for (int k = 0; k < L; ++k)
                     {
-                        const uint32_t v = buffer[k * blockDim.x + (t ^ (1u << bit))];
+                        const uint32_t v = tile.buffer[k * blockDim.x + (t ^ (1u << bit))];
                         lo[k] = upper ? v : lo[k];
                         hi[k] = upper ? hi[k] : v;
                     }
                     // the next exchange writes the other buffer: a thread gets
                     // there only after this barrier's readers of it are done
-                    uint32_t* swap = buffer;
-                    buffer = other;
-                    other = swap;
+                    uint32_t* swap = tile.buffer;
+                    tile.buffer = tile.other;
+                    tile.other = swap;
                 }
             }
             uint32_t next[L];
-            load_twiddle<L>(next, p.twiddles, twiddle_index(j + 1 < w ? j + 1 : j));
+            load_twiddle<L>(next, twiddles, tile.twiddle_index<Inverse>(j + 1 < w ? j + 1 : j));
             if constexpr (!Inverse)
             {
                 mont_mul<L>(hi, hi, tw, m);
@@ -303,11 +271,11 @@ namespace hmpc_gb300
                 {
                     lo[k] = sum[k];
                 }
-                if (p.row_shift + j == p.log_n - 1)
+                if (last && j == w - 1)
                 {
                     // the transform's last stage: tw is T[1], and u + v takes T[0] = N^-1
                     uint32_t scale[L];
-                    load_twiddle<L>(scale, p.twiddles, 0u);
+                    load_twiddle<L>(scale, twiddles, 0u);
                     mont_mul<L>(lo, lo, scale, m);
                 }
                 mont_mul<L>(hi, hi, tw, m);
@@ -318,6 +286,64 @@ namespace hmpc_gb300
                 tw[k] = next[k];
             }
         }
+    }
+
+    // One pass over the tiles of block `block` of the pass's grid.  exchange
+    // holds [2][L][blockDim.x] words.  load and store take the polynomial (within
+    // its part), the index of the lower element of the thread's pair, the
+    // distance to the upper one, and the pair.  Wait: whether the input may
+    // still be being written by the kernel before this one in the stream.
+    // after runs between the stages and the store, in every thread.
+    template<int L, bool Inverse, bool Wait, class Load, class After, class Store>
+    __device__ __forceinline__ void ntt_pair_process(const PairPassParams& p, const Modulus<L>& m, uint64_t block,
+                                                     uint32_t* exchange, Load&& load, After&& after, Store&& store)
+    {
+        const uint32_t t = threadIdx.x;
+        const uint32_t w = p.w, c = p.c;
+        const uint32_t pair_bits = w + c - 1;
+        const uint64_t number = block * (blockDim.x >> pair_bits) + (t >> pair_bits);
+        const bool active = number < p.tiles;
+        const uint32_t col = t & ((1u << c) - 1u);
+        const uint32_t r = (t >> c) & ((1u << (w - 1)) - 1u);  // the row bits but the pair's
+        const uint32_t tile_bits = p.log_n - w - c;
+        uint64_t poly = number >> tile_bits;
+        uint32_t part = 0;
+#pragma unroll
+        for (int i = 1; i < pair_max_parts; ++i)
+        {
+            if (poly >= p.part_polys)
+            {
+                poly -= p.part_polys;
+                ++part;
+            }
+        }
+        const uint32_t in_poly = static_cast<uint32_t>(number) & ((1u << tile_bits) - 1u);
+        const uint32_t mid_bits = p.row_shift - c;
+        const uint32_t high = in_poly >> mid_bits;  // index bits above the rows
+        const uint32_t base = (high << (p.row_shift + w)) | ((in_poly & ((1u << mid_bits) - 1u)) << c) | col;
+        PairTile tile{w, c, r, (1u << (p.log_n - p.row_shift - w)) + high, exchange, exchange + L * blockDim.x};
+        uint32_t lo[L], hi[L], tw[L];
+        load_twiddle<L>(tw, p.twiddles, tile.twiddle_index<Inverse>(0));
+        if constexpr (Wait)
+        {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
+        {
+            const uint32_t row = Inverse ? r << 1 : r;
+            const uint32_t idx = base | (row << p.row_shift);
+            const uint32_t step = 1u << (p.row_shift + (Inverse ? 0u : w - 1));
+            if (active)
+            {
+                load(part, poly, idx, step, lo, hi);
+            }
+            else
+            {
+                set_zero<L>(lo);
+                set_zero<L>(hi);
+            }
+        }
+        pair_stages<L, Inverse>(lo, hi, tw, tile, p.twiddles, p.row_shift + w == p.log_n, m);
+        after(tile, lo, hi);
         // The next kernel's blocks may come in from here on.  Let in at this pass's
         // start they hold slots and issue while they wait: one 4096 pair 13.9 us,
         // a key pair of 2^15 25.4, decryption of 33 x 2^14 81.5; so 12.3, 23.5 and
@@ -357,6 +383,7 @@ namespace hmpc_gb300
                     load1<L>(hi, in + step, p.elements, 0);
                 }
             },
+            [](PairTile&, const uint32_t (&)[L], const uint32_t (&)[L]) {},
             [&](uint32_t part, uint64_t poly, uint32_t idx, uint32_t step, const uint32_t (&lo)[L],
                 const uint32_t (&hi)[L]) {
                 uint32_t* out = p.out[part] + (poly << p.log_n) + idx;
@@ -392,6 +419,7 @@ namespace hmpc_gb300
                 load1<L>(lo, in, d.stride, 0);
                 load1<L>(hi, in + step, d.stride, 0);
             },
+            [](PairTile&, const uint32_t (&)[L], const uint32_t (&)[L]) {},
             [&](uint32_t, uint64_t poly, uint32_t idx, uint32_t step, const uint32_t (&lo)[L],
                 const uint32_t (&hi)[L]) {
                 const PolyRequest& d = p.requests[poly];
@@ -403,7 +431,9 @@ namespace hmpc_gb300
     // Decryption's inverse transform: the first pass forms its input c0 - s * c1
     // (s broadcast over the batch; hmpc/expr/crypto/lhe/dec.hpp:29) as it loads,
     // and the last pass lifts its result to the plaintext modulus (1 or 2 limbs)
-    // as it stores.
+    // before it stores -- for NTT-form plaintexts after the forward transform's
+    // first pass mod p, which works on the same tiles: it starts on the pair bit
+    // that the inverse transform ends on.
     struct DecryptParams
     {
         const uint32_t* s;   // [L][N]
@@ -412,6 +442,7 @@ namespace hmpc_gb300
         uint32_t* out;       // residues mod p, limb planes of `elements`
         CastParams cast;
         uint32_t p[2], pninv;
+        const uint32_t* p_twiddles;  // NTT-form plaintexts: the forward table mod p
     };
 
     // LP: limbs of p in the last pass, 0 in the passes before it
@@ -421,6 +452,8 @@ namespace hmpc_gb300
                                                                               const Modulus<L> m)
     {
         extern __shared__ uint32_t exchange[];
+        uint32_t y[2][LP > 0 ? LP : 1];
+        Modulus<(LP > 0 ? LP : 1)> to;
         ntt_pair_process<L, true, true>(
             p, m, blockIdx.x, exchange,
             [&](uint32_t, uint64_t poly, uint32_t idx, uint32_t step, uint32_t (&lo)[L], uint32_t (&hi)[L]) {
@@ -444,23 +477,39 @@ namespace hmpc_gb300
                     load1<L>(hi, p.out[0], p.elements, at + step);
                 }
             },
-            [&](uint32_t, uint64_t poly, uint32_t idx, uint32_t step, const uint32_t (&lo)[L],
-                const uint32_t (&hi)[L]) {
-                const uint64_t at = (poly << p.log_n) + idx;
+            [&](PairTile& tile, const uint32_t (&lo)[L], const uint32_t (&hi)[L]) {
                 if constexpr (LP > 0)
                 {
-                    Modulus<LP> to;
 #pragma unroll
                     for (int j = 0; j < LP; ++j)
                     {
                         to.q[j] = d.p[j];
                     }
                     to.ninv = d.pninv;
-                    uint32_t y[LP];
-                    cast_value<LP, L>(y, lo, d.cast, to);
-                    store1<LP>(d.out, p.elements, at, y);
-                    cast_value<LP, L>(y, hi, d.cast, to);
-                    store1<LP>(d.out, p.elements, at + step, y);
+                    cast_value<LP, L>(y[0], lo, d.cast, to);
+                    cast_value<LP, L>(y[1], hi, d.cast, to);
+                    if (d.p_twiddles)
+                    {
+                        uint32_t tw[LP];
+                        load_twiddle<LP>(tw, d.p_twiddles, tile.template twiddle_index<false>(0));
+                        pair_stages<LP, false>(y[0], y[1], tw, tile, d.p_twiddles, false, to);
+                    }
+                }
+            },
+            [&](uint32_t, uint64_t poly, uint32_t idx, uint32_t step, const uint32_t (&lo)[L],
+                const uint32_t (&hi)[L]) {
+                uint64_t at = (poly << p.log_n) + idx;
+                if constexpr (LP > 0)
+                {
+                    if (d.p_twiddles)
+                    {
+                        // rows 2r and 2r + 1 in place of r and r + 2^(w-1)
+                        const uint32_t r = (threadIdx.x >> p.c) & ((1u << (p.w - 1)) - 1u);
+                        at += static_cast<uint64_t>(r) << p.row_shift;
+                        step = 1u << p.row_shift;
+                    }
+                    store1<LP>(d.out, p.elements, at, y[0]);
+                    store1<LP>(d.out, p.elements, at + step, y[1]);
                 }
                 else
                 {
