@@ -20,6 +20,7 @@ namespace
     constexpr uint32_t tile_elements = 512;
     constexpr uint32_t tile_max_limbs = 16;  // 33 KB of shared memory, 512 threads
     constexpr uint32_t thread_words = 16;    // 512 * L words over 32 * L threads
+    static_assert(tile_elements == 32 * thread_words, "one warp per limb plane, one keystream block per thread");
 
     __device__ __forceinline__ uint32_t padded(uint32_t w)
     {

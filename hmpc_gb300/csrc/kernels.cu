@@ -412,7 +412,8 @@ namespace hmpc_gb300
             {
                 return cudaSuccess;
             }
-            matvec_kernel<L><<<grid_for(p.total, 256), 256, 0, stream>>>(z, mat, x, p, device_modulus(h));
+            // 128 threads: 119 -> 115 us for 16 x (4 x 4) of degree 2^15 at 8 limbs (shorter last wave)
+            matvec_kernel<L><<<grid_for(p.total, 128), 128, 0, stream>>>(z, mat, x, p, device_modulus(h));
             return cudaGetLastError();
         }
 
@@ -494,10 +495,10 @@ namespace hmpc_gb300
         cudaError_t tc_tail(const TailParams& p, bool encrypt, bool dependent, const HostModulus& h,
                             cudaStream_t stream)
         {
-            const unsigned grid = static_cast<unsigned>(((p.end - p.begin) / 2 + 255) / 256);
+            const unsigned grid = static_cast<unsigned>(((p.end - p.begin) / 2 + 127) / 128);
             const Modulus<L> m = device_modulus(h);
-            return encrypt ? launch(tc_tail_kernel<L, true>, grid, 256, 0, dependent, stream, p, m)
-                           : launch(tc_tail_kernel<L, false>, grid, 256, 0, dependent, stream, p, m);
+            return encrypt ? launch(tc_tail_kernel<L, true>, grid, 128, 0, dependent, stream, p, m)
+                           : launch(tc_tail_kernel<L, false>, grid, 128, 0, dependent, stream, p, m);
         }
 
         cudaError_t ntt_cluster(const ClusterNttParams& p, uint64_t batch, const HostModulus& h, cudaStream_t stream)

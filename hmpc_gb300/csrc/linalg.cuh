@@ -46,7 +46,7 @@ namespace hmpc_gb300
     // vector rows are shared by all `rows` outputs of a batch through L2).  The
     // products are summed unreduced and reduced once.  Bound by the wide
     // multiply-adds and, close behind, HBM: 16 x (4 x 4) of degree 2^15, 8
-    // limbs 158 us with a Montgomery product per term, 119 so (101 G products/s is
+    // limbs 158 us with a Montgomery product per term, 115 so (101 G products/s is
     // this form's rate without the loads, 83 us).
     template<int L>
     __global__ void __launch_bounds__(256) matvec_kernel(uint32_t* z, const uint32_t* mat, const uint32_t* x,

@@ -53,10 +53,11 @@ namespace hmpc_gb300
     // Bound by the wide multiply-adds (their pipe 70 % busy): 1.5 products per
     // element at w = 3, and two more per ciphertext coefficient.  256 encryptions
     // of 2^15 at 8 limbs: 1072 us, against 1001 for the group on the tensor cores
-    // and 355 for the combination after it.  Three blocks per SM (80 registers, a
-    // few spills): 1118 us at two blocks, 1075 at four.
+    // and 355 for the combination after it.  24 warps per SM (80 registers, a few
+    // spills) in blocks of 128: the encryption takes 2737 us, 2769 in blocks of
+    // 256, 2765 at 32 warps, 2815 at 16.
     template<int L, bool Encrypt>
-    __global__ void __launch_bounds__(256, 3) tc_tail_kernel(const TailParams p, const Modulus<L> m)
+    __global__ void __launch_bounds__(128, 6) tc_tail_kernel(const TailParams p, const Modulus<L> m)
     {
         const uint32_t w = p.w;
         const uint64_t id = p.begin / 2 + static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
