@@ -51,8 +51,8 @@ CONFIG = {
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant
 # kernel: the mean over the five tc_group_kernel launches of one fused CBD(10)
 # transform of 256 x 2^15, from the one-pass ncu capture summarised in
-# profiles/tc_group_kernel_cbd_n32768_L8.md (sum of its five launches / 5)
-DOMINANT_TRAFFIC_BYTES = 648.0e6
+# profiles/tc_group_kernel_cbd_n32768_L8.md (sum of its four launches / 4)
+DOMINANT_TRAFFIC_BYTES = 493.8e6
 DOMINANT_TRAFFIC_PROFILE = "profiles/tc_group_kernel_cbd_n32768_L8.md"
 
 
@@ -357,7 +357,8 @@ def dominant_roofline(q, transform_ms, per_transform, int_peak, chacha_peak=None
                         "frac": (first_s + rest_s) / (transform_ms * 1e-3)}
         return {
             "bound": bound,
-            "kernel": "tc_group_kernel (tensor-core transform groups: fused CBD(10) sampler -> NTT, 256 x N=2^15, L=8)",
+            "kernel": "tc_group_kernel (tensor-core transform: fused CBD(10) sampler -> NTT, 256 x N=2^15, L=8; the last "
+                      "three stages in tc_tail_kernel)",
             "achieved": primary["achieved"],
             "peak": primary["peak"],
             "unit": primary["unit"],
@@ -379,7 +380,7 @@ def dominant_roofline(q, transform_ms, per_transform, int_peak, chacha_peak=None
     algorithmic_bytes = 3 * BATCH * N * q.limbs * 4 / per_transform
     return {
         "bound": "int",
-        "kernel": "ntt_pass_kernel (fused CBD(10) sampler -> NTT, 256 x N=2^15, L=8)",
+        "kernel": "ntt_pair_kernel (fused CBD(10) sampler -> NTT, 256 x N=2^15, L=8)",
         "achieved": achieved / 1e12,
         "peak": int_peak / 1e12,
         "unit": "T int32-mul/s",
