@@ -1,9 +1,9 @@
 // Elementwise kernels over limb-planar tensors (limb j of element e at
 // [j * elements + e], hmpc/comp/tensor.hpp:21,25-29).
 //
-// Every thread handles V = 4 consecutive elements so that each limb plane is
-// read and written with 128-bit accesses; HBM traffic is the algorithmic
-// minimum (each operand limb read once, each result limb written once).
+// Every limb plane is read and written with coalesced accesses; HBM traffic is
+// the algorithmic minimum (each operand limb read once, each result limb
+// written once).
 #pragma once
 
 #include <cstdint>
@@ -14,30 +14,69 @@
 
 namespace hmpc_gb300
 {
+    // elements per thread of the reductions
     constexpr int vec = 4;
 
-    template<int L>
-    __device__ __forceinline__ void load4(uint32_t (&x)[vec][L], const uint32_t* t, uint64_t elements, uint64_t e)
+    template<int V>
+    struct VectorWord;
+    template<>
+    struct VectorWord<1>
     {
+        using type = uint32_t;
+    };
+    template<>
+    struct VectorWord<2>
+    {
+        using type = uint2;
+    };
+    template<>
+    struct VectorWord<4>
+    {
+        using type = uint4;
+    };
+
+    // V consecutive elements, one 4 * V-byte access per limb plane: elements
+    // and e are multiples of V, t is aligned to 4 * V bytes
+    template<int L, int V>
+    __device__ __forceinline__ void load_vector(uint32_t (&x)[V][L], const uint32_t* t, uint64_t elements, uint64_t e)
+    {
+        using Word = typename VectorWord<V>::type;
 #pragma unroll
         for (int j = 0; j < L; ++j)
         {
-            const uint4 v = __ldcs(reinterpret_cast<const uint4*>(t + static_cast<uint64_t>(j) * elements + e));
-            x[0][j] = v.x;
-            x[1][j] = v.y;
-            x[2][j] = v.z;
-            x[3][j] = v.w;
+            union
+            {
+                Word v;
+                uint32_t w[V];
+            } word;
+            word.v = __ldcs(reinterpret_cast<const Word*>(t + static_cast<uint64_t>(j) * elements + e));
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+            {
+                x[k][j] = word.w[k];
+            }
         }
     }
 
-    template<int L>
-    __device__ __forceinline__ void store4(uint32_t* t, uint64_t elements, uint64_t e, const uint32_t (&x)[vec][L])
+    template<int L, int V>
+    __device__ __forceinline__ void store_vector(uint32_t* t, uint64_t elements, uint64_t e,
+                                                 const uint32_t (&x)[V][L])
     {
+        using Word = typename VectorWord<V>::type;
 #pragma unroll
         for (int j = 0; j < L; ++j)
         {
-            const uint4 v = make_uint4(x[0][j], x[1][j], x[2][j], x[3][j]);
-            __stcs(reinterpret_cast<uint4*>(t + static_cast<uint64_t>(j) * elements + e), v);
+            union
+            {
+                Word v;
+                uint32_t w[V];
+            } word;
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+            {
+                word.w[k] = x[k][j];
+            }
+            __stcs(reinterpret_cast<Word*>(t + static_cast<uint64_t>(j) * elements + e), word.v);
         }
     }
 
@@ -61,45 +100,47 @@ namespace hmpc_gb300
         }
     }
 
-    // d = a*b + c (examples/fma.cpp:56-67).  vectorised path: elements % 4 == 0
-    // and 16-byte aligned planes; the scalar path covers everything else.
-    template<int L>
-    __global__ void __launch_bounds__(256) fma_kernel(uint32_t* d, const uint32_t* a, const uint32_t* b,
-                                                      const uint32_t* c, uint64_t elements, int vectorised,
-                                                      const Modulus<L> m)
+    // d = a*b + c (examples/fma.cpp:56-67), V elements per thread.  Bound by
+    // memory, which needs many loads in flight: one kernel per width, as one for
+    // all of them had 92 registers at 8 limbs (now 66 for V = 2, 40 for V = 1), and
+    // no loop, in which the compiler delays loads to save registers (8 limbs, V =
+    // 2, 2^24 elements: 348 us with it, 313 without).  8 limbs before and now:
+    // 1500007 elements 47.1 -> 35.0 us (V = 1), 6000000 148 -> 117 us (V = 2, 6.6
+    // TB/s).
+    template<int L, int V>
+    __device__ __forceinline__ void fma_elements(uint32_t* d, const uint32_t* a, const uint32_t* b, const uint32_t* c,
+                                                 uint64_t elements, uint64_t e, const Modulus<L>& m)
     {
-        const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-        if (vectorised)
-        {
-            const uint64_t e = tid * vec;
-            if (e >= elements)
-            {
-                return;
-            }
-            uint32_t x[vec][L], y[vec][L], z[vec][L];
-            load4<L>(x, a, elements, e);
-            load4<L>(y, b, elements, e);
-            load4<L>(z, c, elements, e);
+        uint32_t x[V][L], y[V][L], z[V][L];
+        load_vector<L, V>(x, a, elements, e);
+        load_vector<L, V>(y, b, elements, e);
+        load_vector<L, V>(z, c, elements, e);
 #pragma unroll
-            for (int k = 0; k < vec; ++k)
-            {
-                mont_mul<L>(x[k], x[k], y[k], m);
-                mod_add<L>(x[k], x[k], z[k], m);
-            }
-            store4<L>(d, elements, e, x);
-        }
-        else
+        for (int k = 0; k < V; ++k)
         {
-            for (uint64_t e = tid; e < elements; e += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+            mont_mul<L>(x[k], x[k], y[k], m);
+            mod_add<L>(x[k], x[k], z[k], m);
+        }
+        store_vector<L, V>(d, elements, e, x);
+    }
+
+    template<int L, int V>
+    __global__ void __launch_bounds__(256) fma_kernel(uint32_t* d, const uint32_t* a, const uint32_t* b,
+                                                      const uint32_t* c, uint64_t elements, const Modulus<L> m)
+    {
+        uint64_t e = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * V;
+        if constexpr (L * V == 1)
+        {
+            // one word per thread is bound by the rate of new blocks: they go
+            // on (16777217 elements 57.7 -> 51.3 us)
+            for (; e < elements; e += static_cast<uint64_t>(gridDim.x) * blockDim.x)
             {
-                uint32_t x[L], y[L], z[L];
-                load1<L>(x, a, elements, e);
-                load1<L>(y, b, elements, e);
-                load1<L>(z, c, elements, e);
-                mont_mul<L>(x, x, y, m);
-                mod_add<L>(x, x, z, m);
-                store1<L>(d, elements, e, x);
+                fma_elements<L, V>(d, a, b, c, elements, e, m);
             }
+        }
+        else if (e < elements)
+        {
+            fma_elements<L, V>(d, a, b, c, elements, e, m);
         }
     }
 

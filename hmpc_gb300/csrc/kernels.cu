@@ -1,6 +1,7 @@
 // Per-limb-count kernel instantiations and launchers.  Compiled once per L
 // with -DHMPC_L=<L>; exports kernel_table_<L>().
 #include <algorithm>
+#include <type_traits>
 
 #include "cast.cuh"
 #include "dispatch.hpp"
@@ -119,24 +120,41 @@ namespace hmpc_gb300
         cudaError_t fma(uint32_t* d, const uint32_t* a, const uint32_t* b, const uint32_t* c, uint64_t elements,
                         const HostModulus& h, cudaStream_t stream)
         {
-            const uintptr_t align = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) |
-                                    reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d);
-            const int vectorised = (elements % vec == 0) && (align % 16 == 0);
-            const unsigned block = 256;
-            unsigned grid;
-            if (vectorised)
-            {
-                grid = static_cast<unsigned>((elements / vec + block - 1) / block);
-            }
-            else
-            {
-                grid = grid_for(elements, block);
-            }
             if (elements == 0)
             {
                 return cudaSuccess;
             }
-            fma_kernel<L><<<grid, block, 0, stream>>>(d, a, b, c, elements, vectorised, device_modulus(h));
+            // The widest access that the planes allow, up to two elements per
+            // thread above 4 limbs, where four leave too few warps: 2^24
+            // elements of 8 limbs 354.8 us with four, 313.3 with two, 356.3
+            // with one; of 2 limbs 76.2, 75.9 and 86.1 and 1500008 of them 6.3,
+            // 8.3 and 8.3.  Blocks of 128 threads there (8 limbs, two elements
+            // per thread: 329.7 -> 313.3 us), of 256 below (6000000 elements of
+            // one limb, two per thread: 16.4 -> 14.1 us).
+            constexpr int widest = L <= 4 ? 4 : 2;
+            constexpr unsigned block = L <= 4 ? 256 : 128;
+            const uint64_t shape = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) |
+                                   reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d) | elements * 4;
+            auto launch = [&](auto width) {
+                constexpr int V = decltype(width)::value;
+                const uint64_t threads = elements / V;
+                // only the kernel of single words loops
+                const unsigned grid = L * V == 1 ? grid_for(threads, block)
+                                                 : static_cast<unsigned>((threads + block - 1) / block);
+                fma_kernel<L, V><<<grid, block, 0, stream>>>(d, a, b, c, elements, device_modulus(h));
+            };
+            if (shape % (4 * widest) == 0)
+            {
+                launch(std::integral_constant<int, widest>{});
+            }
+            else if (shape % 8 == 0)
+            {
+                launch(std::integral_constant<int, 2>{});
+            }
+            else
+            {
+                launch(std::integral_constant<int, 1>{});
+            }
             return cudaGetLastError();
         }
 

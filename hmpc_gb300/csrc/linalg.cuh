@@ -309,7 +309,7 @@ namespace hmpc_gb300
             for (uint64_t e = tid * vec; e < elements; e += threads * vec)
             {
                 uint32_t x[vec][L];
-                load4<L>(x, in, elements, e);
+                load_vector<L, vec>(x, in, elements, e);
 #pragma unroll
                 for (int k = 0; k < vec; ++k)
                 {
