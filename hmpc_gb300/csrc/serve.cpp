@@ -418,8 +418,11 @@ struct hmpc_server
                     ++failed;
                 }
             }
+            // under the lock: between a drain's look at the count and its wait, a
+            // change and its notification would be missed, and the drain sleep
+            // until its timeout
+            in_system.fetch_sub(d.reqs.size());
         }
-        in_system.fetch_sub(d.reqs.size());
         if (d.bytes)
         {
             pool.release(d.offset, d.bytes);
@@ -706,10 +709,10 @@ int hmpc_server_submit(hmpc_server* srv, const hmpc_request* request, uint64_t* 
         x->ticket = srv->next_ticket++;
         *ticket = x->ticket;
         ++srv->submitted;
+        srv->in_system.fetch_add(1);  // before the worker can see, and finish, the request
         srv->incoming.push_back(x.get());
         srv->requests.emplace(x->ticket, std::move(x));
     }
-    srv->in_system.fetch_add(1);
     srv->cv.notify_all();
     return HMPC_OK;
 }
