@@ -279,6 +279,8 @@ namespace hmpc_gb300::detail
                       const PolyRequest* requests = nullptr, uint32_t rng_slot = 0, bool cuda_cores_only = false);
     int run_plain(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t batch, bool inverse, int kind,
                   uint32_t vx2, uint32_t security, const uint32_t* src, uint32_t* out);
+    // whether two runs of device words share one
+    bool overlap(const uint32_t* a, uint64_t a_words, const uint32_t* b, uint64_t b_words);
     CastParams make_cast(const hmpc_modulus* dst, const hmpc_modulus* src);
     bool capturing(const hmpc_context* ctx);
     // whether an encryption's (or key pair's) transforms run as parts of one set

@@ -119,11 +119,53 @@ namespace
         uint64_t total_ = 0;
     };
 
+    // Device words held as disjoint ascending ranges.
+    class Ranges
+    {
+    public:
+        void clear()
+        {
+            ranges_.clear();
+        }
+        bool overlaps(const uint32_t* words, uint64_t count)
+        {
+            const auto it = ending_after(words);
+            return it != ranges_.end() && it->first < words + count;
+        }
+        void add(const uint32_t* words, uint64_t count)
+        {
+            const uint32_t* end = words + count;
+            const auto first = ending_after(words);
+            auto last = first;
+            for (; last != ranges_.end() && last->first < end; ++last)
+            {
+                words = std::min(words, last->first);
+                end = std::max(end, last->second);
+            }
+            ranges_.insert(ranges_.erase(first, last), {words, end});
+        }
+
+    private:
+        using Range = std::pair<const uint32_t*, const uint32_t*>;
+        std::vector<Range>::iterator ending_after(const uint32_t* words)
+        {
+            return std::upper_bound(ranges_.begin(), ranges_.end(), words,
+                                    [](const uint32_t* w, const Range& r) { return w < r.second; });
+        }
+        std::vector<Range> ranges_;
+    };
+
     struct Dispatch
     {
         std::vector<Request*> reqs;
         int lane = -1;
         uint64_t offset = 0, bytes = 0;
+        // No request writes what another one reads or writes, so they may run side
+        // by side in their own buffers.  Otherwise (a transform submitted twice into
+        // one buffer, a result over another request's input) a pass of one would
+        // meet half-made results of another: every input is gathered before the
+        // first result is written, and the results follow in the requests' order.
+        bool apart = true;
     };
 
     using GroupKey = std::tuple<int, const void*, uint64_t, uint32_t>;  // kind, modulus, n, key
@@ -144,6 +186,7 @@ struct hmpc_server
     uint8_t* pool_base = nullptr;
     Pool pool;
     std::vector<ResidentKey> keys;
+    Ranges read_words, written_words;        // of the dispatch being put together (worker thread)
 
     std::mutex mu;
     std::condition_variable cv;
@@ -210,6 +253,41 @@ struct hmpc_server
             w += words_of(k.p, k.n, polys) + 2 * words_of(k.q, k.n, polys);  // plaintext, c0, c1
         }
         return w;
+    }
+
+    // whether the dispatch's requests stay apart with one more
+    bool stays_apart(const Dispatch& d, const hmpc_request& r)
+    {
+        if (!d.apart || r.kind == HMPC_REQUEST_CT_MUL)
+        {
+            return d.apart;  // products are one launch each, in order
+        }
+        const uint64_t out_words = words_of(r.q, r.n, r.count);
+        const bool encrypt = r.kind == HMPC_REQUEST_ENCRYPT;
+        const uint64_t in_words = encrypt ? words_of(keys[r.key_id].p, r.n, r.count) : out_words;
+        bool apart = !written_words.overlaps(r.in0, in_words);
+        for (const uint32_t* out : {r.out0, encrypt ? r.out1 : nullptr})
+        {
+            apart = apart && !(out && (written_words.overlaps(out, out_words) || read_words.overlaps(out, out_words)));
+        }
+        // a transform may run in place, but not over a part of its own input
+        return apart && (encrypt || r.out0 == r.in0 || !overlap(r.out0, out_words, r.in0, in_words));
+    }
+
+    void joined(const hmpc_request& r)
+    {
+        if (r.kind == HMPC_REQUEST_CT_MUL)
+        {
+            return;
+        }
+        const uint64_t out_words = words_of(r.q, r.n, r.count);
+        const bool encrypt = r.kind == HMPC_REQUEST_ENCRYPT;
+        read_words.add(r.in0, encrypt ? words_of(keys[r.key_id].p, r.n, r.count) : out_words);
+        written_words.add(r.out0, out_words);
+        if (encrypt)
+        {
+            written_words.add(r.out1, out_words);
+        }
     }
 
     GroupKey group_of(const hmpc_request& r) const
@@ -296,17 +374,20 @@ struct hmpc_server
             {
                 return run_transform(lane, q, r0.n, r0.count, false, producer_tensor, 0, 0, r0.in0, r0.out0);
             }
-            // between the requests' own buffers, unless their plan is an engine
-            // that works on one buffer
-            const PolyRequest* dev_desc = nullptr;
-            if (int rc = describe(d, r0.n, polys, &dev_desc))
+            // between the requests' own buffers, unless these are not apart or
+            // the plan is an engine that works on one buffer
+            if (d.apart)
             {
-                return rc;
-            }
-            bool done = false;
-            if (int rc = run_requests(lane, q, r0.n, polys, dev_desc, done); rc || done)
-            {
-                return rc;
+                const PolyRequest* dev_desc = nullptr;
+                if (int rc = describe(d, r0.n, polys, &dev_desc))
+                {
+                    return rc;
+                }
+                bool done = false;
+                if (int rc = run_requests(lane, q, r0.n, polys, dev_desc, done); rc || done)
+                {
+                    return rc;
+                }
             }
             const uint64_t total = r0.n * polys;
             uint64_t at = 0;
@@ -360,7 +441,7 @@ struct hmpc_server
         {
             return rc;
         }
-        if (parts_applicable(k.q, k.p))
+        if (d.apart && parts_applicable(k.q, k.p))
         {
             return encrypt_cuda_cores(lane, k.q, k.p, n, polys, k.a, k.b, nullptr, nullptr, nullptr, scratch, dev_desc,
                                       false);
@@ -500,6 +581,8 @@ struct hmpc_server
                 }
                 Dispatch d;
                 d.lane = lane;
+                read_words.clear();
+                written_words.clear();
                 uint64_t polys = 0;
                 while (!best->empty() && d.reqs.size() < max_batch &&
                        polys + best->front()->r.count <= desc_capacity)
@@ -528,6 +611,8 @@ struct hmpc_server
                     }
                     d.offset = offset;
                     d.bytes = need;
+                    d.apart = stays_apart(d, best->front()->r);
+                    joined(best->front()->r);
                     polys += best->front()->r.count;
                     best->pop_front();
                 }

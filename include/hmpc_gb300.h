@@ -444,7 +444,11 @@ int hmpc_server_create(hmpc_context* ctx, const hmpc_server_config* config, hmpc
  * server copies it */
 int hmpc_server_add_key(hmpc_server* server, hmpc_modulus* q, hmpc_modulus* p, uint64_t n, const uint32_t* a,
                         const uint32_t* b, uint32_t* key_id);
-/* non-blocking; the buffers must stay valid until the request is done */
+/* Non-blocking; the buffers must stay valid until the request is done.
+ * Requests of one dispatch may share buffers (its inputs are read before its
+ * results are written, results in the requests' order); dispatches in flight on
+ * different lanes run side by side, so a buffer that one of them writes belongs
+ * to no other until its request is done. */
 int hmpc_server_submit(hmpc_server* server, const hmpc_request* request, uint64_t* ticket);
 /* state: HMPC_REQUEST_*; latency_us (may be NULL): submit -> completion */
 int hmpc_server_poll(hmpc_server* server, uint64_t ticket, int* state, double* latency_us);
