@@ -479,14 +479,12 @@ namespace hmpc_gb300::detail
         return HMPC_OK;
     }
 
-    int run_requests(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t polys, const PolyRequest* requests,
-                     bool& done)
+    int run_requests(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t polys, const PolyRequest* requests)
     {
-        const hmpc_modulus::TileChoice choice = mod->choice(n, false, polys);
-        done = choice.radix_bits >= 2;
-        if (!done)
+        hmpc_modulus::TileChoice choice = mod->choice(n, false, polys);
+        if (choice.radix_bits < 2)
         {
-            return HMPC_OK;
+            choice = hmpc_modulus::TileChoice{};
         }
         Tables* t = nullptr;
         if (int rc = mod->prepare(n, &t))

@@ -295,9 +295,8 @@ namespace hmpc_gb300::detail
                            const uint32_t* key_a, const uint32_t* key_b, const uint32_t* coefficients, uint32_t* c0,
                            uint32_t* c1, uint32_t* workspace, const PolyRequest* requests, bool cuda_cores_only);
     // forward transforms of `polys` polynomials of degree n between the requests'
-    // own buffers, if the shape's plan is a CUDA-core one (else done = false)
-    int run_requests(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t polys, const PolyRequest* requests,
-                     bool& done);
+    // own buffers, on the CUDA cores
+    int run_requests(hmpc_context* ctx, hmpc_modulus* mod, uint64_t n, uint64_t polys, const PolyRequest* requests);
     // tensor-core engine: whether the modulus qualifies (2 to 8 limbs, q
     // below 0.996 * 2^(32L), top limb at least 32) and whether a call does
     // (forward from a tensor or CBD(V) samples, or inverse; at least 16

@@ -160,6 +160,8 @@ namespace
         std::vector<Request*> reqs;
         int lane = -1;
         uint64_t offset = 0, bytes = 0;
+        uint64_t own_words = 0, tc_words = 0;  // of the scratch: buffers of its own, tensor-core digits after them
+        bool direct = false;                   // runs in the requests' own buffers
         // No request writes what another one reads or writes, so they may run side
         // by side in their own buffers.  Otherwise (a transform submitted twice into
         // one buffer, a result over another request's input) a pass of one would
@@ -220,9 +222,19 @@ struct hmpc_server
         return 2 * ((4ull * static_cast<uint64_t>(q->c.limbs) + 5) / 4) * n * polys;
     }
 
-    // scratch bytes of a dispatch of the given requests: buffers of its own
-    // and, after them, the digit buffers of a tensor-core transform
-    uint64_t scratch_bytes(const std::vector<Request*>& rs) const
+    // What a dispatch of the given requests takes, and which way it then runs:
+    // a plan that changes before it is issued does not change the dispatch.
+    struct Need
+    {
+        uint64_t own = 0, tc = 0;  // words
+        bool direct = false;
+        uint64_t bytes() const
+        {
+            return (own + tc) * 4;
+        }
+    };
+
+    Need need_of(const std::vector<Request*>& rs, bool apart) const
     {
         const hmpc_request& r0 = rs.front()->r;
         uint64_t polys = 0;
@@ -231,28 +243,26 @@ struct hmpc_server
             polys += x->r.count;
         }
         const bool single = rs.size() == 1;
-        switch (r0.kind)
+        Need need;
+        if (r0.kind == HMPC_REQUEST_NTT)
         {
-        case HMPC_REQUEST_NTT:
-            return ((single ? 0 : words_of(r0.q, r0.n, polys)) + tc_words(r0.q, r0.n, polys)) * 4;
-        case HMPC_REQUEST_ENCRYPT:
+            need.direct = !single && apart && r0.q->choice(r0.n, false, polys).radix_bits >= 2;
+            need.own = single || need.direct ? 0 : words_of(r0.q, r0.n, polys);
+            need.tc = need.direct ? 0 : tc_words(r0.q, r0.n, polys);
+        }
+        else if (r0.kind == HMPC_REQUEST_ENCRYPT)
         {
             const ResidentKey& k = keys[r0.key_id];
-            return (encrypt_words(k, polys, single) + tc_words(k.q, k.n, polys)) * 4;
+            const bool parts = parts_applicable(k.q, k.p);
+            need.direct = parts && apart;
+            need.own = 3 * words_of(k.q, k.n, polys);  // u, v/w, msg
+            if (!single && !need.direct)
+            {
+                need.own += words_of(k.p, k.n, polys) + 2 * words_of(k.q, k.n, polys);  // plaintext, c0, c1
+            }
+            need.tc = parts ? 0 : tc_words(k.q, k.n, polys);
         }
-        default:
-            return 0;
-        }
-    }
-
-    static uint64_t encrypt_words(const ResidentKey& k, uint64_t polys, bool single)
-    {
-        uint64_t w = 3 * words_of(k.q, k.n, polys);  // u, v/w, msg
-        if (!single)
-        {
-            w += words_of(k.p, k.n, polys) + 2 * words_of(k.q, k.n, polys);  // plaintext, c0, c1
-        }
-        return w;
+        return need;
     }
 
     // whether the dispatch's requests stay apart with one more
@@ -354,17 +364,10 @@ struct hmpc_server
                 ctx->tc_lent_words = 0;
             }
         } lend{lane};
-        if (r0.kind == HMPC_REQUEST_NTT || r0.kind == HMPC_REQUEST_ENCRYPT)
+        if (d.tc_words)
         {
-            const bool ntt = r0.kind == HMPC_REQUEST_NTT;
-            hmpc_modulus* q = ntt ? r0.q : keys[r0.key_id].q;
-            const uint64_t n = ntt ? r0.n : keys[r0.key_id].n;
-            const uint64_t own = ntt ? (single ? 0 : words_of(q, n, polys)) : encrypt_words(keys[r0.key_id], polys, single);
-            if (const uint64_t tw = tc_words(q, n, polys))
-            {
-                lane->tc_lent = scratch + own;
-                lane->tc_lent_words = tw;
-            }
+            lane->tc_lent = scratch + d.own_words;
+            lane->tc_lent_words = d.tc_words;
         }
         if (r0.kind == HMPC_REQUEST_NTT)
         {
@@ -376,18 +379,14 @@ struct hmpc_server
             }
             // between the requests' own buffers, unless these are not apart or
             // the plan is an engine that works on one buffer
-            if (d.apart)
+            if (d.direct)
             {
                 const PolyRequest* dev_desc = nullptr;
                 if (int rc = describe(d, r0.n, polys, &dev_desc))
                 {
                     return rc;
                 }
-                bool done = false;
-                if (int rc = run_requests(lane, q, r0.n, polys, dev_desc, done); rc || done)
-                {
-                    return rc;
-                }
+                return run_requests(lane, q, r0.n, polys, dev_desc);
             }
             const uint64_t total = r0.n * polys;
             uint64_t at = 0;
@@ -441,7 +440,7 @@ struct hmpc_server
         {
             return rc;
         }
-        if (d.apart && parts_applicable(k.q, k.p))
+        if (d.direct)
         {
             return encrypt_cuda_cores(lane, k.q, k.p, n, polys, k.a, k.b, nullptr, nullptr, nullptr, scratch, dev_desc,
                                       false);
@@ -588,8 +587,9 @@ struct hmpc_server
                        polys + best->front()->r.count <= desc_capacity)
                 {
                     d.reqs.push_back(best->front());
-                    const uint64_t need = scratch_bytes(d.reqs);
-                    if (need > pool.total())
+                    const bool apart = stays_apart(d, best->front()->r);
+                    const Need need = need_of(d.reqs, apart);
+                    if (need.bytes() > pool.total())
                     {
                         d.reqs.pop_back();
                         break;
@@ -600,7 +600,7 @@ struct hmpc_server
                         pool.release(d.offset, d.bytes);
                     }
                     uint64_t offset = 0;
-                    if (need && !pool.allocate(need, offset))
+                    if (need.bytes() && !pool.allocate(need.bytes(), offset))
                     {
                         if (d.bytes)
                         {
@@ -610,8 +610,11 @@ struct hmpc_server
                         break;
                     }
                     d.offset = offset;
-                    d.bytes = need;
-                    d.apart = stays_apart(d, best->front()->r);
+                    d.bytes = need.bytes();
+                    d.own_words = need.own;
+                    d.tc_words = need.tc;
+                    d.direct = need.direct;
+                    d.apart = apart;
                     joined(best->front()->r);
                     polys += best->front()->r.count;
                     best->pop_front();
@@ -786,7 +789,7 @@ int hmpc_server_submit(hmpc_server* srv, const hmpc_request* request, uint64_t* 
         std::lock_guard<std::mutex> lock(srv->mu);
         // a request that cannot run even alone is rejected
         std::vector<Request*> alone{x.get()};
-        if (srv->scratch_bytes(alone) > srv->pool.total())
+        if (srv->need_of(alone, true).bytes() > srv->pool.total())
         {
             ++srv->rejected;
             return fail(HMPC_ERROR_REJECTED, "request needs more scratch than the server's memory budget");
