@@ -433,14 +433,15 @@ namespace hmpc_gb300::detail
     // batch (or from the requests' with that slot) and goes to out[i].
     int run_parts(hmpc_context* ctx, hmpc_modulus* q, const hmpc_modulus* p, uint64_t n, uint64_t batch, int count,
                   const uint32_t* kinds, const uint32_t* slots, uint32_t* const* out, const uint32_t* msg,
-                  const PolyRequest* requests)
+                  const PolyRequest* requests, const hmpc_modulus::TileChoice& choice)
     {
         Tables* t = nullptr;
         if (int rc = q->prepare(n, &t))
         {
             return rc;
         }
-        const std::vector<PairPlan> plan = plan_pairs(q->c.limbs, __builtin_ctzll(n), batch * count, false, 0, 0);
+        const std::vector<PairPlan> plan =
+            plan_pairs(q->c.limbs, __builtin_ctzll(n), batch * count, false, choice.local_bits, choice.col_bits);
         const bool dependent = !capturing(ctx);
         for (size_t i = 0; i < plan.size(); ++i)
         {
@@ -530,7 +531,15 @@ namespace hmpc_gb300::detail
             const uint32_t kinds[3] = {part_ternary, part_scaled_message, part_scaled};
             const uint32_t slots[3] = {0, 1, 2};
             uint32_t* const outs[3] = {u, v, msg};
-            if (int rc = run_parts(ctx, q, p, n, batch, 3, kinds, slots, outs, coefficients, requests))
+            // In the shape set or tuned for the transforms of (n, batch), three times
+            // as many polynomials here: 16 of 2^14 at 8 limbs 152 us by the rule, 142
+            // tuned; 8 of 2^13 43.5 and 45.7, the largest loss met.
+            hmpc_modulus::TileChoice choice = q->choice(n, false, batch);
+            if (choice.radix_bits < 2)
+            {
+                choice = hmpc_modulus::TileChoice{};
+            }
+            if (int rc = run_parts(ctx, q, p, n, batch, 3, kinds, slots, outs, coefficients, requests, choice))
             {
                 return rc;
             }
@@ -1508,7 +1517,10 @@ int hmpc_lhe_keygen(hmpc_context* ctx, hmpc_modulus* q, hmpc_modulus* p, uint64_
         const uint32_t kinds[2] = {part_ternary, part_scaled};
         const uint32_t slots[2] = {1, 2};
         uint32_t* const outs[2] = {s, e_poly};
-        if (int rc = run_parts(ctx, q, p, n, 1, 2, kinds, slots, outs, nullptr, nullptr))
+        // by the rule for two polynomials, whatever is set for one: the tiles that
+        // spread one polynomial over the SMs are a pass too many for two (2^15 at 8
+        // limbs 18.4 us by the rule, 24.6 in the shape tuned for one)
+        if (int rc = run_parts(ctx, q, p, n, 1, 2, kinds, slots, outs, nullptr, nullptr, hmpc_modulus::TileChoice{}))
         {
             return rc;
         }

@@ -111,8 +111,13 @@ int hmpc_modulus_root(hmpc_modulus* mod, uint64_t n, int inverse, uint32_t* root
  * cluster of 8 CTAs per polynomial holding it in distributed shared memory,
  * one launch per transform (degrees 2^10..2^14, tensor producer; other calls
  * run the default tiles).  No counterpart in the reference (its transform
- * has one schedule).  hmpc_modulus_tune times the candidates on the device
- * (scratch buffers, values irrelevant to the cost) and keeps the fastest. */
+ * has one schedule).  An encryption on the CUDA cores runs its transforms in
+ * the forward tiles of (degree, batch); a decryption whose inverse transform
+ * runs in tiles, p of one or two limbs and below q, starts the transform mod p in
+ * the same tiles; a key pair's two polynomials take the tiles of the rule where
+ * p has one or two limbs and q at least 72 bits.  hmpc_modulus_tune times the
+ * candidates on the device (scratch buffers, values irrelevant to the cost) and
+ * keeps the fastest. */
 int hmpc_modulus_set_plan(hmpc_modulus* mod, uint64_t n, uint64_t batch, int inverse, int radix_bits, int local_bits,
                           int col_bits);
 int hmpc_modulus_tune(hmpc_modulus* mod, uint64_t n, uint64_t batch, int inverse, float* best_ms);
