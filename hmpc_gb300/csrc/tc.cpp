@@ -636,6 +636,7 @@ namespace hmpc_gb300::detail
             p.w = tt->groups.back().g;
             p.out = out;
             p.out_polys = out_polys;
+            p.error = ctx->tc_error;
             if (combine)
             {
                 p.key_a = combine->key_a;

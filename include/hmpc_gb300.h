@@ -67,7 +67,8 @@ int hmpc_context_set_nonce(hmpc_context* ctx, const uint32_t nonce[3]);
 int hmpc_context_launch_count(const hmpc_context* ctx, uint64_t* count);
 /* hmpc::comp::queue::wait (hmpc/comp/queue.hpp:531-534).  Also reports
  * HMPC_ERROR_TIMEOUT when a tensor-core transform launched since the last
- * call gave up one of its bounded waits (and clears that state). */
+ * call gave up one of its bounded waits (and clears that state); the outputs of
+ * tensor-core transforms launched since then are incomplete or left as they were. */
 int hmpc_context_synchronize(hmpc_context* ctx);
 /* Test hook for the bounded waits of the tensor-core transform (no
  * counterpart in the reference): every wait of its group kernels gives up
