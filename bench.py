@@ -211,6 +211,25 @@ def whole_job_rate(units_per_rank, world, steps, elapsed_ms):
     return world * units_per_rank * steps / (elapsed_ms * 1e-3)
 
 
+def double_buffered(count, load, encrypt, read):
+    """Enqueues `count` steps over two buffer sets: step i is loaded, encrypted
+    and read back in set i % 2.  The encryption of step i goes first, then the
+    read of step i - 1, then the load of step i + 1: each copy waits for an
+    encryption that was enqueued before the next one, so the copies overlap the
+    following encryption even where the device takes all streams' work through
+    one queue in enqueue order.  Returns the set that holds the last step's
+    result."""
+    load(0)
+    for i in range(count):
+        encrypt(i)
+        if i > 0:
+            read(i - 1)
+        if i + 1 < count:
+            load(i + 1)
+    read(count - 1)
+    return (count - 1) % 2
+
+
 def dist_setup():
     world = int(os.environ.get("WORLD_SIZE", "1"))
     rank = int(os.environ.get("RANK", "0"))
@@ -1007,12 +1026,6 @@ def main():
     # and copies both ciphertext halves back, as a serving loop does: the
     # copies of one step overlap the encryption of the next (a copy-in and a
     # copy-out stream, two buffer sets; events order the reuse of each set).
-
-    # Host enqueue order per step i: the encryption of step i, then the
-    # copy-out of step i - 1, then the copy-in of step i + 1.  Each copy waits
-    # for an encryption that was enqueued before the next one, so the copies
-    # overlap the following encryption even where the device takes all
-    # streams' work through one queue in enqueue order.
     def load(i):
         b = sets[i % 2]
         copy_in.wait_event(b["done"])  # the set's plaintexts are no longer read
@@ -1036,22 +1049,12 @@ def main():
             b["c1"].copy_(b["ct"].c1.data, non_blocking=True)
         b["read"].record(copy_out)
 
-    def e2e_run(count):
-        load(0)
-        for i in range(count):
-            encrypt(i)
-            if i > 0:
-                read(i - 1)
-            if i + 1 < count:
-                load(i + 1)
-        read(count - 1)
-
-    e2e_run(args.warmup)
+    double_buffered(args.warmup, load, encrypt, read)
     barrier()
     e_start, e_stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e_start.record(stream)
     copy_in.wait_stream(stream)
-    e2e_run(args.steps)
+    last = sets[double_buffered(args.steps, load, encrypt, read)]
     stream.wait_stream(copy_out)
     e_stop.record(stream)
     barrier()
@@ -1068,19 +1071,21 @@ def main():
         with ClockSampler(local) as es_clocks:
             es_start.record(stream)
             copy_in.wait_stream(stream)
-            e2e_run(count)
+            last = sets[double_buffered(count, load, encrypt, read)]
             stream.wait_stream(copy_out)
             es_stop.record(stream)
             barrier()
         es_ms = max_over_ranks(es_start.elapsed_time(es_stop), world, device="cuda")
         e2e_sustained = {"steps": count, "value": whole_job_rate(BATCH, world, count, es_ms),
                          "clocks": es_clocks.summary()}
-    last = sets[(args.steps - 1) % 2]
     host_c0, host_c1 = last["c0"], last["c1"]
-    # check the e2e result once: decrypting the copied-back ciphertext gives the messages
+    # check the e2e result once: decrypting the copied-back ciphertext of the
+    # last step that ran (each step has a key pair of its own) gives the messages
     back = lhe.Ciphertext(Tensor(q, (BATCH,), N, host_c0.to(queue.device)), Tensor(q, (BATCH,), N,
                                                                                host_c1.to(queue.device)))
     ok = bool((lhe.dec(queue, s, back, p).data == msgs.data).all().item())
+    if not ok:
+        sys.exit("end to end: the copied-back ciphertexts do not decrypt to the messages")
     # the host link's pinned copy rates on this machine, each direction alone on
     # its copy stream: the copies of a step bound e2e at BATCH / max(in, out)
     link = {}
