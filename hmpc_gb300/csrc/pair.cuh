@@ -201,14 +201,15 @@ namespace hmpc_gb300
     // The stages of a pass on the pair (lo, hi), tw the first stage's twiddle; by
     // every thread of the block.  last: the inverse transform's last stage is the
     // pass's last.
-    template<int L, bool Inverse>
-    __device__ __forceinline__ void pair_stages(uint32_t (&lo)[L], uint32_t (&hi)[L], uint32_t (&tw)[L],
+    // W: the pass's stages where the loop is unrolled, 0: as many as the tile says.
+    template<int L, bool Inverse, int W>
+    __device__ __forceinline__ void pair_stage_loop(uint32_t (&lo)[L], uint32_t (&hi)[L], uint32_t (&tw)[L],
                                                 PairTile& tile, const uint32_t* twiddles, bool last,
                                                 const Modulus<L>& m)
     {
         const uint32_t t = threadIdx.x;
-        const uint32_t w = tile.w;
-#pragma unroll 1
+        const uint32_t w = W ? W : tile.w;
+#pragma unroll(W ? W : 1)
         for (uint32_t j = 0; j < w; ++j)
         {
             if (j > 0)
@@ -286,6 +287,35 @@ namespace hmpc_gb300
                 tw[k] = next[k];
             }
         }
+    }
+
+    // One and two limbs: the stages' own code, their indices and exchanges, takes
+    // more of the issue slots (80 % busy) than the products, so the loop is
+    // unrolled, one copy for each number of stages.  128 of 2^15, forward and
+    // inverse: 73 and 83 us -> 60 and 62 at one limb, 117 and 124 -> 107 and 108 at
+    // two.  With more limbs the products hide that code, and copies of them would
+    // outgrow the instruction cache.
+    template<int L, bool Inverse>
+    __device__ __forceinline__ void pair_stages(uint32_t (&lo)[L], uint32_t (&hi)[L], uint32_t (&tw)[L],
+                                                PairTile& tile, const uint32_t* twiddles, bool last,
+                                                const Modulus<L>& m)
+    {
+        if constexpr (L <= 2)
+        {
+            switch (tile.w)
+            {
+            case 3: return pair_stage_loop<L, Inverse, 3>(lo, hi, tw, tile, twiddles, last, m);
+            case 4: return pair_stage_loop<L, Inverse, 4>(lo, hi, tw, tile, twiddles, last, m);
+            case 5: return pair_stage_loop<L, Inverse, 5>(lo, hi, tw, tile, twiddles, last, m);
+            case 6: return pair_stage_loop<L, Inverse, 6>(lo, hi, tw, tile, twiddles, last, m);
+            case 7: return pair_stage_loop<L, Inverse, 7>(lo, hi, tw, tile, twiddles, last, m);
+            case 8: return pair_stage_loop<L, Inverse, 8>(lo, hi, tw, tile, twiddles, last, m);
+            case 9: return pair_stage_loop<L, Inverse, 9>(lo, hi, tw, tile, twiddles, last, m);
+            case 10: return pair_stage_loop<L, Inverse, 10>(lo, hi, tw, tile, twiddles, last, m);
+            default: break;
+            }
+        }
+        pair_stage_loop<L, Inverse, 0>(lo, hi, tw, tile, twiddles, last, m);
     }
 
     // One pass over the tiles of block `block` of the pass's grid.  exchange
@@ -492,7 +522,7 @@ namespace hmpc_gb300
                     {
                         uint32_t tw[LP];
                         load_twiddle<LP>(tw, d.p_twiddles, tile.template twiddle_index<false>(0));
-                        pair_stages<LP, false>(y[0], y[1], tw, tile, d.p_twiddles, false, to);
+                        pair_stage_loop<LP, false, 0>(y[0], y[1], tw, tile, d.p_twiddles, false, to);
                     }
                 }
             },
