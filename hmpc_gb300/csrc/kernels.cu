@@ -431,7 +431,16 @@ namespace hmpc_gb300
                 return cudaSuccess;
             }
             // 128 threads: 119 -> 115 us for 16 x (4 x 4) of degree 2^15 at 8 limbs (shorter last wave)
-            matvec_kernel<L><<<grid_for(p.total, 128), 128, 0, stream>>>(z, mat, x, p, device_modulus(h));
+            const unsigned grid = grid_for(p.total, 128);
+            // lazily where there are products to add up (figures at the kernel)
+            if (L > 1 && p.cols > 1)
+            {
+                matvec_kernel<L, (L > 1)><<<grid, 128, 0, stream>>>(z, mat, x, p, device_modulus(h));
+            }
+            else
+            {
+                matvec_kernel<L, false><<<grid, 128, 0, stream>>>(z, mat, x, p, device_modulus(h));
+            }
             return cudaGetLastError();
         }
 

@@ -47,8 +47,12 @@ namespace hmpc_gb300
     // products are summed unreduced and reduced once.  Bound by the wide
     // multiply-adds and, close behind, HBM: 16 x (4 x 4) of degree 2^15, 8
     // limbs 158 us with a Montgomery product per term, 115 so (101 G products/s is
-    // this form's rate without the loads, 83 us).
-    template<int L>
+    // this form's rate without the loads, 83 us).  Lazy: so; else a Montgomery
+    // product per term, for single columns, where there is nothing to add up
+    // (16 x (1 x 1) of 2^15, 4 limbs 10.3 us lazily, 8.2 so), and for single words,
+    // where it is the loads in flight that count (one 3000 x 3000 matrix 247 and
+    // 162 us).
+    template<int L, bool Lazy>
     __global__ void __launch_bounds__(256) matvec_kernel(uint32_t* z, const uint32_t* mat, const uint32_t* x,
                                                          const MatvecParams p, const Modulus<L> m)
     {
@@ -58,13 +62,25 @@ namespace hmpc_gb300
             const MatvecIndex ix = matvec_index(p, e);
             const uint64_t mb = ix.b * p.m_bstride + ix.i * p.cols * p.coeffs + ix.c;
             const uint64_t xb = ix.b * p.x_bstride + ix.c;
-            uint32_t acc[2 * L], a[L], v[L];
-            set_zero<2 * L>(acc);
-            if (p.cols)
+            uint32_t a[L], v[L];
+            if constexpr (!Lazy)
             {
-                load1<L>(a, mat, p.m_elements, mb);
-                load1<L>(v, x, p.x_elements, xb);
+                uint32_t sum[L];
+                set_zero<L>(sum);
+                for (uint64_t k = 0; k < p.cols; ++k)
+                {
+                    load1<L>(a, mat, p.m_elements, mb + k * p.coeffs);
+                    load1<L>(v, x, p.x_elements, xb + k * p.coeffs);
+                    mont_mul<L>(a, a, v, m);
+                    mod_add<L>(sum, sum, a, m);
+                }
+                store1<L>(z, p.total, e, sum);
+                continue;
             }
+            uint32_t acc[2 * L];
+            set_zero<2 * L>(acc);
+            load1<L>(a, mat, p.m_elements, mb);
+            load1<L>(v, x, p.x_elements, xb);
 #pragma unroll 1
             for (uint64_t k = 0; k < p.cols; ++k)
             {
