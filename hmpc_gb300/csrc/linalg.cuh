@@ -308,9 +308,10 @@ namespace hmpc_gb300
     // `out` (limb-planar, out_elements = the number of blocks).  The second
     // level is this kernel on the block values with one block.  The operations
     // are associative and commutative on exact values, so the grouping does
-    // not change the result.
+    // not change the result.  Three limbs at 32 registers, eight blocks per SM,
+    // where the compiler takes 34: a product of 10,000,001 residues 66 -> 51 us.
     template<int L, bool Mod>
-    __global__ void __launch_bounds__(256) reduce_kernel(uint32_t* out, uint64_t out_elements, const uint32_t* in,
+    __global__ void __launch_bounds__(256, Mod && L == 3 ? 8 : 1) reduce_kernel(uint32_t* out, uint64_t out_elements, const uint32_t* in,
                                                          uint64_t elements, bool vectorised,
                                                          const Reducer<L, Mod> red)
     {
