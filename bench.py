@@ -49,9 +49,9 @@ CONFIG = {
     "l2": "per-step working set 640 MiB (messages 64 MiB + ciphertexts 512 MiB + intermediates) > 129 MB L2",
 }
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant
-# kernel: the mean over the five tc_group_kernel launches of one fused CBD(10)
-# transform of 256 x 2^15, from the one-pass ncu capture summarised in
-# profiles/tc_group_kernel_cbd_n32768_L8.md (sum of its four launches / 4)
+# kernel: the mean over the four launches (the wide group, two groups, the last
+# stages) of one fused CBD(10) transform of 256 x 2^15, from the one-pass ncu
+# capture summarised in profiles/tc_group_kernel_cbd_n32768_L8.md
 DOMINANT_TRAFFIC_BYTES = 493.8e6
 DOMINANT_TRAFFIC_PROFILE = "profiles/tc_group_kernel_cbd_n32768_L8.md"
 

@@ -1006,6 +1006,9 @@ int hmpc_modulus_set_plan(hmpc_modulus* mod, uint64_t n, uint64_t batch, int inv
         local_bits = 0;
         col_bits = 0;
     }
+    // Tiles of up to ten bits are what runs, and all of them fit; more bits run as
+    // ten, and are refused where a tile that held as many in shared memory would
+    // not have fitted, so that the statuses stay what they were.
     else if ((radix_bits != 2 && radix_bits != 3) || local_bits < 0 || local_bits > 13 || col_bits < 0 ||
              col_bits > 6 ||
              (local_bits && static_cast<uint64_t>(mod->c.limbs) * 4u * ((33u << local_bits) >> 5) > 200 * 1024))

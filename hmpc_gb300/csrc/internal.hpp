@@ -208,10 +208,11 @@ struct hmpc_modulus
         }
     }
 
-    // tile shape per (log2 N, inverse, batch): register radix bits, tile
-    // bits, column bits -- set by hmpc_modulus_tune / hmpc_modulus_set_plan.
-    // Radix bits 0 selects the tensor-core engine; its local_bits is the output
-    // split (1 or 2; 0 = 1) of the group whose rows are contiguous.
+    // tile shape per (log2 N, inverse, batch): radix bits, tile bits (0: the
+    // rule's shape), column bits -- set by hmpc_modulus_tune /
+    // hmpc_modulus_set_plan.  Radix bits 2 and 3 both are the CUDA-core tiles, 1 the
+    // cluster, 0 the tensor-core engine; its local_bits is the output split (1 or 2;
+    // 0 = 1) of the group whose rows are contiguous.
     struct TileChoice
     {
         int radix_bits = 3;

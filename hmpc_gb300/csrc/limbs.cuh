@@ -183,7 +183,10 @@ namespace hmpc_gb300
     // a_j * b lies exactly on one 64-bit column, so a row of products is two
     // chains of mad.lo.cc / madc.hi.cc pairs over adjacent words; each pair is
     // one wide multiply-add with carry in and out, where a single running sum
-    // needs a further addition for each product.
+    // needs a further addition for each product.  Keeping the sums of even and odd
+    // columns apart is a known way to whole carry chains (Emmart, Luitjens, Weems
+    // and Woolley, "Optimizing Modular Multiplication for NVIDIA's Maxwell GPUs",
+    // ARITH 2016, does it for 16-bit products).
     template<int L>
     struct Columns
     {

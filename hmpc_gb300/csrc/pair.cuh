@@ -15,7 +15,7 @@
 // lies in the warp, through shared memory otherwise.
 //
 // Bound by the wide multiply-adds of the butterflies' products where the
-// polynomials fill the SMs (256 of 2^15 at 8 limbs: 1154 us, 0.82 of the
+// polynomials fill the SMs (256 of 2^15 at 8 limbs: 1154 us, 0.76 of the
 // product rate), by the latency of the stages where they do not.  One
 // butterfly per thread and one copy of the product's code in the stage loop:
 // holding 8 elements in registers and unrolling three stages of butterflies

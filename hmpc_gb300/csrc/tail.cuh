@@ -28,8 +28,6 @@
 
 namespace hmpc_gb300
 {
-    constexpr int tail_max_stages = 6;
-
     struct TailParams
     {
         const uint32_t* digits;   // [L + 1][stride] words of four biased digits
@@ -53,7 +51,7 @@ namespace hmpc_gb300
 
     // Bound by the wide multiply-adds (their pipe 70 % busy): 1.5 products per
     // element at w = 3, and two more per ciphertext coefficient.  256 encryptions
-    // of 2^15 at 8 limbs: 1072 us, against 1001 for the group on the tensor cores
+    // of 2^15 at 8 limbs: 1050 us, against 1001 for the group on the tensor cores
     // and 355 for the combination after it.  24 warps per SM (80 registers, a few
     // spills) in blocks of 128: the encryption takes 2737 us, 2769 in blocks of
     // 256, 2765 at 32 warps, 2815 at 16.

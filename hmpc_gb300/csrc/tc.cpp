@@ -18,9 +18,12 @@ namespace
         return tc_kernels(mod->c.limbs);
     }
 
-    // launches of a transform's groups of up to three stages; a transform with a
-    // tail keeps the number (the tail takes the launches of the groups it
-    // replaces, a share of the elements each)
+    // Launches of a transform's groups of up to three stages.  A transform with a
+    // tail keeps the number, which hmpc_tc_cost and the launch counter report: the
+    // tail takes the launches of the groups it replaces, a share of the elements
+    // each.  That is no gain: the shares run one after another.  One launch for all
+    // of them takes 0.2 % less at 256 encryptions of 2^15 (8 limbs) and 20 % less at
+    // 16 of 2^14 (202 -> 160 us).
     int group_launches(int log_n)
     {
         return (log_n + 2) / 3;
@@ -667,7 +670,7 @@ namespace hmpc_gb300::detail
             const bool dependent = cudaStreamIsCapturing(stream, &capture) == cudaSuccess &&
                                    capture == cudaStreamCaptureStatusNone;
             // the launches of the groups it replaces, and of an encryption's
-            // combination (one for polynomials in buffers of their own)
+            // combination (group_launches); one for polynomials in buffers of their own
             const uint64_t launches =
                 out_polys ? 1
                           : static_cast<uint64_t>(group_launches(static_cast<int>(log_n))) - (tt->groups.size() - 1) +
