@@ -180,6 +180,7 @@ struct hmpc_server
     std::vector<std::unique_ptr<hmpc_context>> lanes;
     std::vector<cudaEvent_t> lane_done;
     std::vector<PolyRequest*> lane_desc;     // pinned descriptors per lane
+    uint32_t* lane_error = nullptr;          // pinned, one per lane: its tensor-core error word after a dispatch
     std::vector<Dispatch> lane_work;
     std::vector<bool> lane_busy;
     uint32_t desc_capacity = 0;              // polynomials per lane descriptor buffer
@@ -353,6 +354,8 @@ struct hmpc_server
             polys += x->r.count;
         }
         uint32_t* scratch = reinterpret_cast<uint32_t*>(pool_base + d.offset);
+        lane->tc_spin_limit = ctx->tc_spin_limit;
+        lane->tc_test_stall = ctx->tc_test_stall;
         // the lane's tensor-core digit buffers come from the dispatch's share
         // of the pool, after its own buffers
         struct Lend
@@ -478,9 +481,26 @@ struct hmpc_server
         return HMPC_OK;
     }
 
+    // the lane's error word, on its way to the host behind the dispatch's work
+    cudaError_t report(int lane_index)
+    {
+        hmpc_context* lane = lanes[static_cast<size_t>(lane_index)].get();
+        return lane->tc_error ? cudaMemcpyAsync(lane_error + lane_index, lane->tc_error, sizeof(uint32_t),
+                                                cudaMemcpyDeviceToHost, lane->stream)
+                              : cudaSuccess;
+    }
+
     void finish(int lane_index, bool ok)
     {
         Dispatch& d = lane_work[static_cast<size_t>(lane_index)];
+        if (lane_error[lane_index])
+        {
+            // a bounded wait ran out: the requests failed, the next dispatch starts clean
+            ok = false;
+            lane_error[lane_index] = 0;
+            hmpc_context* lane = lanes[static_cast<size_t>(lane_index)].get();
+            cudaMemsetAsync(lane->tc_error, 0, sizeof(uint32_t), lane->stream);
+        }
         const auto now = clock_type::now();
         {
             std::lock_guard<std::mutex> lock(mu);
@@ -632,8 +652,12 @@ struct hmpc_server
                 ++dispatches;
                 batched_requests += d.reqs.size();
                 const int rc = issue(lane_work[static_cast<size_t>(lane)]);
-                const cudaError_t e = cudaEventRecord(lane_done[static_cast<size_t>(lane)],
-                                                      lanes[static_cast<size_t>(lane)]->stream);
+                cudaError_t e = report(lane);
+                if (e == cudaSuccess)
+                {
+                    e = cudaEventRecord(lane_done[static_cast<size_t>(lane)],
+                                        lanes[static_cast<size_t>(lane)]->stream);
+                }
                 if (rc != HMPC_OK || e != cudaSuccess)
                 {
                     cudaStreamSynchronize(lanes[static_cast<size_t>(lane)]->stream);
@@ -681,6 +705,8 @@ int hmpc_server_create(hmpc_context* ctx, const hmpc_server_config* config, hmpc
         srv->lane_done.push_back(ev);
         srv->lane_desc.push_back(desc);
     }
+    HMPC_CUDA(cudaMallocHost(&srv->lane_error, config->lanes * sizeof(uint32_t)), "allocating the lanes' error words");
+    std::fill(srv->lane_error, srv->lane_error + config->lanes, 0u);
     srv->lane_work.resize(config->lanes);
     srv->lane_busy.assign(config->lanes, false);
     HMPC_CUDA(cudaMalloc(&srv->d_desc, srv->desc_capacity * static_cast<uint64_t>(config->lanes) * sizeof(PolyRequest)),
@@ -902,6 +928,7 @@ int hmpc_server_destroy(hmpc_server* srv)
         cudaFree(k.a);
         cudaFree(k.b);
     }
+    cudaFreeHost(srv->lane_error);
     cudaFree(srv->d_desc);
     cudaFree(srv->pool_base);
     delete srv;

@@ -78,7 +78,8 @@ int hmpc_context_synchronize(hmpc_context* ctx);
  * that wait runs out: every launch returns early with its output incomplete,
  * having waited for its copies in flight and freed its tensor memory, and
  * hmpc_context_synchronize reports HMPC_ERROR_TIMEOUT.  stall = 0 restores
- * normal operation; the context stays usable throughout. */
+ * normal operation; the context stays usable throughout.  A server on the
+ * context follows it, and reports the requests as failed. */
 int hmpc_context_set_test_wait(hmpc_context* ctx, uint32_t polls, int stall);
 
 /* --- moduli ---------------------------------------------------------------
@@ -436,7 +437,7 @@ typedef struct hmpc_request
 #define HMPC_REQUEST_QUEUED 0
 #define HMPC_REQUEST_RUNNING 1
 #define HMPC_REQUEST_DONE 2
-#define HMPC_REQUEST_FAILED (-2)
+#define HMPC_REQUEST_FAILED (-2) /* a launch failed, or a tensor-core transform gave up a bounded wait */
 
 typedef struct hmpc_server_stats
 {
